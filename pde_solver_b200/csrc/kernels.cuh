@@ -935,68 +935,10 @@ __device__ __forceinline__ double ext_value(const GridDev& gc, const TC* __restr
   return coef == 0.0 ? 0.0 : coef * double(xc[cidx(gc, I, J, K)]);
 }
 
-// Trilinear (bilinear in 2D) interpolation of the coarse correction, extended
-// to the coarse boundary through the closures, added to the fine interior.
-template <typename T, typename TC>
-__global__ void __launch_bounds__(kBx* kBy) k_prolong_add(GridDev gf, GridDev gc, const TC* __restrict__ xc,
-                                                          T* __restrict__ xf, const Ctl* ctl) {
-  if (ctl_skip_dep(ctl)) return;
-  const int i = blockIdx.x * kBx + threadIdx.x;
-  const int j = blockIdx.y * kBy + threadIdx.y;
-  int k0, k1;
-  column_range(gf, k0, k1);
-  if (!(i >= 1 && i <= gf.nx - 2 && j >= 1 && j <= gf.ny - 2)) return;
-  int I0, J0;
-  double tx, ty;
-  coarse_pos(i, gf.nx, gc.nx, map_mode(gf.nx, gc.nx), I0, tx);
-  coarse_pos(j, gf.ny, gc.ny, map_mode(gf.ny, gc.ny), J0, ty);
-  const int I1 = tx != 0.0 ? I0 + 1 : I0, J1 = ty != 0.0 ? J0 + 1 : J0;
-  const bool xy_edge = I0 == 0 || I1 == gc.nx - 1 || J0 == 0 || J1 == gc.ny - 1;
-  const int zmode = gf.dim == 3 ? map_mode(gf.nz, gc.nz) : 0;
-  for (int k = k0; k < k1; ++k) {
-    int K0 = 0, K1 = 0;
-    double tz = 0.0;
-    if (gf.dim == 3) {
-      coarse_pos(k, gf.nz, gc.nz, zmode, K0, tz);
-      K1 = tz != 0.0 ? K0 + 1 : K0;
-    }
-    double c000, c100, c010, c110, c001, c101, c011, c111;
-    if (!xy_edge && !(gf.dim == 3 && (K0 == 0 || K1 == gc.nz - 1))) {
-      const long long a0 = (long long)K0 * gc.sxy, a1 = (long long)K1 * gc.sxy;
-      const long long r0 = (long long)J0 * gc.nx, r1 = (long long)J1 * gc.nx;
-      c000 = double(xc[a0 + r0 + I0]);
-      c100 = double(xc[a0 + r0 + I1]);
-      c010 = double(xc[a0 + r1 + I0]);
-      c110 = double(xc[a0 + r1 + I1]);
-      c001 = double(xc[a1 + r0 + I0]);
-      c101 = double(xc[a1 + r0 + I1]);
-      c011 = double(xc[a1 + r1 + I0]);
-      c111 = double(xc[a1 + r1 + I1]);
-    } else {
-      c000 = ext_value(gc, xc, I0, J0, K0);
-      c100 = ext_value(gc, xc, I1, J0, K0);
-      c010 = ext_value(gc, xc, I0, J1, K0);
-      c110 = ext_value(gc, xc, I1, J1, K0);
-      c001 = ext_value(gc, xc, I0, J0, K1);
-      c101 = ext_value(gc, xc, I1, J0, K1);
-      c011 = ext_value(gc, xc, I0, J1, K1);
-      c111 = ext_value(gc, xc, I1, J1, K1);
-    }
-    const double x00 = (1.0 - tx) * c000 + tx * c100, x10 = (1.0 - tx) * c010 + tx * c110;
-    const double x01 = (1.0 - tx) * c001 + tx * c101, x11 = (1.0 - tx) * c011 + tx * c111;
-    const double y0 = (1.0 - ty) * x00 + ty * x10, y1 = (1.0 - ty) * x01 + ty * x11;
-    const double v = (1.0 - tz) * y0 + tz * y1;
-    const long long id = ((long long)k * gf.ny + j) * gf.nx + i;
-    xf[id] = T(double(xf[id]) + v);
-  }
-}
-
-// z-marching transfer kernels for level pairs whose z map is the identity or
-// nested 2:1 (every odd side, and every 2D grid). One thread per column:
-// restriction sums each fine plane's x-y weights once and shares the plane
-// sum between the two coarse planes it feeds; prolongation evaluates the
-// bilinear x-y interpolation once per coarse plane and reuses it for the 2-3
-// fine planes it feeds (same expressions as k_prolong_add, so the same bits).
+// z-marching restriction for level pairs whose z map is the identity or
+// nested 2:1 (every odd side, and every 2D grid). One thread per column sums
+// each fine plane's x-y weights once and shares the plane sum between the two
+// coarse planes it feeds.
 __device__ __forceinline__ bool z_marchable(const GridDev& gf, const GridDev& gc) {
   return gf.dim != 3 || map_mode(gf.nz, gc.nz) <= 1;
 }
@@ -1078,72 +1020,138 @@ __global__ void __launch_bounds__(kBx* kBy) k_restrict_march(GridDev gf, GridDev
   }
 }
 
-template <typename T, typename TC>
-__global__ void __launch_bounds__(kBx* kBy) k_prolong_march(GridDev gf, GridDev gc, const TC* __restrict__ xc,
-                                                            T* __restrict__ xf, const Ctl* ctl) {
+// Level sizes of a transfer, without the face descriptors of GridDev (700
+// bytes of kernel parameters per grid that the transfers do not read).
+struct LevelGeo {
+  int nx, ny, nz, dim;
+  long long sxy;
+};
+
+inline LevelGeo level_geo(const GridDev& g) { return LevelGeo{g.nx, g.ny, g.nz, g.dim, g.sxy}; }
+
+// Extension of a coarse correction to the coarse boundary in separable form.
+// The homogeneous closure chain of a boundary node (ext_chain) multiplies one
+// factor c1 per face it lies on, and is 0 on a Dirichlet face; with one c1
+// per face the value at (I, J, K) is therefore ax(I) ay(J) az(K) times the
+// value at the indices clamped to the interior, with a(0) = lo, a(n-1) = hi
+// and 1 inside. No thread then walks a chain of face tests.
+struct ExtCoef {
+  double lo[3], hi[3];
+};
+
+// false when a Neumann/Robin face of g carries per-node c1 values (Robin
+// alpha or beta arrays): the chains are then evaluated node by node.
+inline bool ext_coef(const GridDev& g, ExtCoef* e) {
+  bool scalar = true;
+  for (int a = 0; a < 3; ++a) {
+    double* v[2] = {&e->lo[a], &e->hi[a]};
+    for (int m = 0; m < 2; ++m) {
+      const FaceDev& f = g.face[2 * a + m];
+      *v[m] = f.active && f.kind != kDirichlet ? f.c1.s : 0.0;
+      if (f.active && f.kind != kDirichlet && f.c1.a) scalar = false;
+    }
+  }
+  return scalar;
+}
+
+__device__ __forceinline__ double ext_axis(const ExtCoef& e, int a, int I, int n) {
+  return I == 0 ? e.lo[a] : (I == n - 1 ? e.hi[a] : 1.0);
+}
+__device__ __forceinline__ int ext_clamp(int I, int n) { return I < 1 ? 1 : (I > n - 2 ? n - 2 : I); }
+
+// The node-by-node form behind the scalar one (ARR instantiations), out of line.
+template <typename TC>
+__device__ __noinline__ double ext_value_arr(const GridDev& gc, const TC* __restrict__ xc, int I, int J, int K) {
+  return ext_value(gc, xc, I, J, K);
+}
+
+// Prolongation-add for any level pair: trilinear (bilinear in 2D)
+// interpolation of the coarse correction, extended to the coarse boundary
+// through the closures, added to the fine interior. A thread owns a fine
+// column and marches in z, keeping the bilinear x-y value of the two coarse
+// planes around it; four planes are loaded before any is stored. The boundary
+// extension is branch-free (ExtCoef); walking the closure chain of every
+// corner of an edge column in line made the small levels instruction-bound:
+// 8.8 -> 3.9 us per launch on the levels of a 100x77x58 grid, 2.5 -> 2.0 us on
+// those of a 257x193 grid (launches of 1 MB and less, bound by latency).
+template <typename T, typename TC, bool ARR>
+__global__ void __launch_bounds__(kBx* kBy) k_prolong(LevelGeo gf, LevelGeo gc, ExtCoef e, GridDev gcf,
+                                                      const TC* __restrict__ xc, T* __restrict__ xf,
+                                                      const Ctl* ctl) {
   if (ctl_skip_dep(ctl)) return;
-  const int i = blockIdx.x * kBx + threadIdx.x;
-  const int j = blockIdx.y * kBy + threadIdx.y;
-  int k0, k1;
-  column_range(gf, k0, k1);
-  if (!(i >= 1 && i <= gf.nx - 2 && j >= 1 && j <= gf.ny - 2) || k0 >= k1) return;
-  int I0, J0;
-  double tx, ty;
+  const int i = 1 + blockIdx.x * kBx + threadIdx.x;
+  const int j = 1 + blockIdx.y * kBy + threadIdx.y;
+  const bool is3 = gf.dim == 3;
+  const int kb = is3 ? 1 : 0, ke = is3 ? gf.nz - 1 : 1;
+  const int chunk = (ke - kb + gridDim.z - 1) / gridDim.z;
+  const int k0 = kb + blockIdx.z * chunk, k1 = min(ke, k0 + chunk);
+  if (i > gf.nx - 2 || j > gf.ny - 2 || k0 >= k1) return;
+  int I0, J0, Kc = 0;
+  double tx, ty, tz = 0.0;
   coarse_pos(i, gf.nx, gc.nx, map_mode(gf.nx, gc.nx), I0, tx);
   coarse_pos(j, gf.ny, gc.ny, map_mode(gf.ny, gc.ny), J0, ty);
   const int I1 = tx != 0.0 ? I0 + 1 : I0, J1 = ty != 0.0 ? J0 + 1 : J0;
-  const bool xy_edge = I0 == 0 || I1 == gc.nx - 1 || J0 == 0 || J1 == gc.ny - 1;
-  const int zmode = gf.dim == 3 ? map_mode(gf.nz, gc.nz) : 0;
-  // bilinear value on coarse plane K (boundary values through the closures)
+  const double ax0 = ext_axis(e, 0, I0, gc.nx), ax1 = ext_axis(e, 0, I1, gc.nx);
+  const double ay0 = ext_axis(e, 1, J0, gc.ny), ay1 = ext_axis(e, 1, J1, gc.ny);
+  const double w00 = ay0 * ax0, w10 = ay0 * ax1, w01 = ay1 * ax0, w11 = ay1 * ax1;
+  const int cx0 = ext_clamp(I0, gc.nx), cx1 = ext_clamp(I1, gc.nx);
+  const int cy0 = ext_clamp(J0, gc.ny) * gc.nx, cy1 = ext_clamp(J1, gc.ny) * gc.nx;
   auto bilinear = [&](int K) -> double {
     double c00, c10, c01, c11;
-    if (!xy_edge && !(gf.dim == 3 && (K == 0 || K == gc.nz - 1))) {
-      const long long a = (long long)K * gc.sxy;
-      const long long r0 = (long long)J0 * gc.nx, r1 = (long long)J1 * gc.nx;
-      c00 = double(xc[a + r0 + I0]);
-      c10 = double(xc[a + r0 + I1]);
-      c01 = double(xc[a + r1 + I0]);
-      c11 = double(xc[a + r1 + I1]);
+    if constexpr (ARR) {
+      c00 = ext_value_arr(gcf, xc, I0, J0, K);
+      c10 = ext_value_arr(gcf, xc, I1, J0, K);
+      c01 = ext_value_arr(gcf, xc, I0, J1, K);
+      c11 = ext_value_arr(gcf, xc, I1, J1, K);
     } else {
-      c00 = ext_value(gc, xc, I0, J0, K);
-      c10 = ext_value(gc, xc, I1, J0, K);
-      c01 = ext_value(gc, xc, I0, J1, K);
-      c11 = ext_value(gc, xc, I1, J1, K);
+      const double az = is3 ? ext_axis(e, 2, K, gc.nz) : 1.0;
+      const TC* p = xc + (is3 ? (long long)ext_clamp(K, gc.nz) * gc.sxy : 0);
+      const double v00 = double(p[cy0 + cx0]), v10 = double(p[cy0 + cx1]);
+      const double v01 = double(p[cy1 + cx0]), v11 = double(p[cy1 + cx1]);
+      c00 = az * w00 * v00;
+      c10 = az * w10 * v10;
+      c01 = az * w01 * v01;
+      c11 = az * w11 * v11;
     }
     const double x0 = (1.0 - tx) * c00 + tx * c10, x1 = (1.0 - tx) * c01 + tx * c11;
     return (1.0 - ty) * x0 + ty * x1;
   };
-  int ka = -1, kb = -1;
-  double va = 0.0, vb = 0.0;
-  auto at = [&](int K) -> double {
-    if (K == ka) return va;
-    if (K == kb) return vb;
-    const double v = bilinear(K);
-    ka = kb;
-    va = vb;
-    kb = K;
-    vb = v;
-    return v;
-  };
-  // groups of four planes: the four fine values are loaded before any is
-  // stored, so a thread has four loads in flight instead of one
+  T* col = xf + ((long long)k0 * gf.ny + j) * gf.nx + i;
+  if (!is3) {
+    const double y = bilinear(0);
+    *col = T(double(*col) + y);
+    return;
+  }
+  const int zmode = map_mode(gf.nz, gc.nz);
+  // coarse interval of plane k and its remainder, advanced without divisions
+  const int m = gc.nz - 1, den = gf.nz - 1;
+  Kc = zmode == 0 ? k0 : (zmode == 1 ? k0 >> 1 : (k0 * m) / den);
+  int rem = k0 * m - Kc * den;
+  double ya = bilinear(Kc), yb = bilinear(min(Kc + 1, gc.nz - 1));
+  int Ka = Kc;  // ya, yb: planes Ka, Ka + 1
   constexpr int kGroup = 4;
-  for (int kg = k0; kg < k1; kg += kGroup) {
+  for (int kg = k0; kg < k1; kg += kGroup, col += kGroup * gf.sxy) {
     T old[kGroup];
 #pragma unroll
     for (int q = 0; q < kGroup; ++q)
-      if (kg + q < k1) old[q] = xf[((long long)(kg + q) * gf.ny + j) * gf.nx + i];
+      if (kg + q < k1) old[q] = col[q * gf.sxy];
 #pragma unroll
     for (int q = 0; q < kGroup; ++q) {
-      const int k = kg + q;
-      if (k >= k1) break;
-      int K0 = 0;
-      double tz = 0.0;
-      if (gf.dim == 3) coarse_pos(k, gf.nz, gc.nz, zmode, K0, tz);
-      const double y0 = at(K0);
-      const double y1 = tz != 0.0 ? at(K0 + 1) : y0;
-      const double v = (1.0 - tz) * y0 + tz * y1;
-      xf[((long long)k * gf.ny + j) * gf.nx + i] = T(double(old[q]) + v);
+      if (kg + q < k1) {
+        if (Ka != Kc) {
+          ya = yb;
+          Ka = Kc;
+          yb = bilinear(min(Kc + 1, gc.nz - 1));
+        }
+        tz = double(rem) / double(den);
+        const double v = (1.0 - tz) * ya + tz * (rem ? yb : ya);
+        col[q * gf.sxy] = T(double(old[q]) + v);
+      }
+      rem += m;
+      if (rem >= den) {
+        rem -= den;
+        ++Kc;
+      }
     }
   }
 }
@@ -1153,12 +1161,14 @@ __global__ void __launch_bounds__(kBx* kBy) k_prolong_march(GridDev gf, GridDev 
 // it interpolates to, and marches over a chunk of coarse planes K, writing fine
 // planes 2K and 2K+1. The four coarse values of a plane are loaded once for
 // the four columns, and the eight fine values of a step are loaded before
-// any is stored; the arithmetic of every fine node is that of
-// k_prolong_march (same weights and expressions, so the same bits). At 257^3:
-// 68 against 98.5 us per launch stand-alone.
-template <typename T, typename TC>
-__global__ void __launch_bounds__(kBx* kBy) k_prolong_pair(GridDev gf, GridDev gc, const TC* __restrict__ xc,
-                                                           T* __restrict__ xf, const Ctl* ctl) {
+// any is stored; the weights of every fine node are those of k_prolong. At
+// 257^3: 68 against 98.5 us per launch of a thread per fine column
+// stand-alone; with the branch-free extension instead of the closure chains
+// the five levels of a 257^3 V-cycle take 66 instead of 83 us.
+template <typename T, typename TC, bool ARR>
+__global__ void __launch_bounds__(kBx* kBy) k_prolong_pair(LevelGeo gf, LevelGeo gc, ExtCoef e, GridDev gcf,
+                                                           const TC* __restrict__ xc, T* __restrict__ xf,
+                                                           const Ctl* ctl) {
   if (ctl_skip_dep(ctl)) return;
   const int I = blockIdx.x * kBx + threadIdx.x;
   const int J = blockIdx.y * kBy + threadIdx.y;
@@ -1167,22 +1177,33 @@ __global__ void __launch_bounds__(kBx* kBy) k_prolong_pair(GridDev gf, GridDev g
   const int chunk = (nK + gridDim.z - 1) / gridDim.z;
   const int Ka = blockIdx.z * chunk, Kb = min(nK, Ka + chunk);
   if (Ka >= Kb) return;
+  const double ax0 = ext_axis(e, 0, I, gc.nx), ax1 = ext_axis(e, 0, I + 1, gc.nx);
+  const double ay0 = ext_axis(e, 1, J, gc.ny), ay1 = ext_axis(e, 1, J + 1, gc.ny);
   const bool xy_edge = I == 0 || I + 1 == gc.nx - 1 || J == 0 || J + 1 == gc.ny - 1;
+  const int cx0 = ext_clamp(I, gc.nx), cx1 = ext_clamp(I + 1, gc.nx);
+  const int cy0 = ext_clamp(J, gc.ny) * gc.nx, cy1 = ext_clamp(J + 1, gc.ny) * gc.nx;
   // bilinear values of the four fine columns on coarse plane K (boundary
-  // values through the closures, as in k_prolong_march)
+  // values through the closures, as in k_prolong)
   auto bil4 = [&](int K, double (&y)[4]) {
     double C00, C10, C01, C11;
-    if (!xy_edge && !(K == 0 || K == gc.nz - 1)) {
-      const long long a = (long long)K * gc.sxy + (long long)J * gc.nx + I;
-      C00 = double(xc[a]);
-      C10 = double(xc[a + 1]);
-      C01 = double(xc[a + gc.nx]);
-      C11 = double(xc[a + gc.nx + 1]);
+    if constexpr (ARR) {
+      C00 = ext_value_arr(gcf, xc, I, J, K);
+      C10 = ext_value_arr(gcf, xc, I + 1, J, K);
+      C01 = ext_value_arr(gcf, xc, I, J + 1, K);
+      C11 = ext_value_arr(gcf, xc, I + 1, J + 1, K);
     } else {
-      C00 = ext_value(gc, xc, I, J, K);
-      C10 = ext_value(gc, xc, I + 1, J, K);
-      C01 = ext_value(gc, xc, I, J + 1, K);
-      C11 = ext_value(gc, xc, I + 1, J + 1, K);
+      const TC* p = xc + (long long)ext_clamp(K, gc.nz) * gc.sxy;
+      C00 = double(p[cy0 + cx0]);
+      C10 = double(p[cy0 + cx1]);
+      C01 = double(p[cy1 + cx0]);
+      C11 = double(p[cy1 + cx1]);
+      if (xy_edge || K == 0 || K == gc.nz - 1) {
+        const double az = ext_axis(e, 2, K, gc.nz);
+        C00 *= az * (ay0 * ax0);
+        C10 *= az * (ay0 * ax1);
+        C01 *= az * (ay1 * ax0);
+        C11 *= az * (ay1 * ax1);
+      }
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {

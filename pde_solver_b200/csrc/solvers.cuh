@@ -420,6 +420,19 @@ inline dim3 prolong_pair_grid(const GridDev& gc) {
   return dim3(xy.x, xy.y, (unsigned)chunks);
 }
 
+// launch shape of k_prolong: 32 x 8 interior fine columns per block, z chunks
+// of at least four planes (its load group) for about 148 x 8 blocks
+inline dim3 prolong_grid(const GridDev& g) {
+  const dim3 xy((g.nx - 2 + kBx - 1) / kBx, (g.ny - 2 + kBy - 1) / kBy, 1);
+  const long long xyb = (long long)xy.x * xy.y;
+  const int kint = g.dim == 3 ? g.nz - 2 : 1;
+  long long chunks = (148LL * 8 + xyb - 1) / xyb;
+  if (chunks > (kint + 3) / 4) chunks = (kint + 3) / 4;
+  if (chunks > kMaxGridBlocks / xyb) chunks = kMaxGridBlocks / xyb;
+  if (chunks < 1) chunks = 1;
+  return dim3(xy.x, xy.y, (unsigned)chunks);
+}
+
 template <typename KT>
 inline void inject_k(Context* ctx, const GridDev& gf, const GridDev& gc, const KT* kf, KT* kc) {
   k_inject<KT><<<vec_blocks(gc.n, ctx), 256, 0, ctx->stream>>>(gf, gc, kf, kc);
@@ -790,17 +803,16 @@ struct Hierarchy {
     level(ctx, l + 1, rhs0, ctl);
     {
       ProfScope ps(ctx, "prolong_add", l, dofs * sizeof(T) * (2.0 + 1.0 / (L.g.dim == 3 ? 8.0 : 4.0)));
+      ExtCoef e;
+      const bool scalar = ext_coef(C.g, &e);
+      const LevelGeo gf = level_geo(L.g), gc = level_geo(C.g);
       if (nested_3d(L.g, C.g))
-        launch_dep(ctx, prolong_pair_grid(C.g), stencil_block(), 0, k_prolong_pair<T, T>, L.g, C.g, (const T*)C.out,
-                   cur, ctl);
-      else if (z_nested(L.g, C.g))
-        // 148*24 target blocks (12 z chunks at 257^3): 101.7 -> 97 us against
-        // 148*16; 148*12 and 148*40 are slower
-        launch_dep(ctx, stencil_grid_auto(L.g, 148 * 24), stencil_block(), 0, k_prolong_march<T, T>, L.g, C.g,
+        launch_dep(ctx, prolong_pair_grid(C.g), stencil_block(), 0,
+                   scalar ? k_prolong_pair<T, T, false> : k_prolong_pair<T, T, true>, gf, gc, e, C.g,
                    (const T*)C.out, cur, ctl);
       else
-        launch_dep(ctx, stencil_grid_auto(L.g), stencil_block(), 0, k_prolong_add<T, T>, L.g, C.g, (const T*)C.out,
-                   cur, ctl);
+        launch_dep(ctx, prolong_grid(L.g), stencil_block(), 0, scalar ? k_prolong<T, T, false> : k_prolong<T, T, true>,
+                   gf, gc, e, C.g, (const T*)C.out, cur, ctl);
     }
     ctx->count();
     if (l == 0 && dot_slot && post > 0 && L.march) {
