@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/pdeb200.h"
+#include "cluster.cuh"
 #include "kernels.cuh"
 
 namespace pdeb {
@@ -267,6 +268,31 @@ inline void launch_dep(const Context* ctx, dim3 grid, dim3 block, size_t smem, v
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = ctx->pdl ? 1 : 0;
+  PDEB_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
+}
+
+// Launch of a cluster kernel (cluster.cuh): one cluster of cs.csize CTAs. The
+// attributes are the same constants for every launch of a kernel, so threads
+// that launch it at once do not disturb each other.
+constexpr size_t kClusterDynSmem = kClusterSmem - 10 * 1024;  // the kernels' static shared memory stays below 10 KB
+
+template <typename... KArgs, typename... Args>
+inline void launch_cluster(const Context* ctx, const ClusterShape& cs, size_t smem, void (*kern)(KArgs...),
+                           Args&&... args) {
+  PDEB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterDynSmem));
+  PDEB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cs.csize);
+  cfg.blockDim = dim3(cs.threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cs.csize;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   PDEB_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
 }
 

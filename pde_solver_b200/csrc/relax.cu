@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "cluster.cuh"
 #include "host.h"
 #include "solvers.cuh"
 
@@ -186,6 +187,282 @@ __global__ void __launch_bounds__(1024) k_gs_lex_block(GridDev g, Coef cf, const
   }
 }
 
+// ------------------------------------------ lexicographic Gauss-Seidel / SOR
+
+constexpr int kLexSweeps = 512;   // sweeps of a batch (tested together)
+
+struct ClusterLexArgs {
+  const double* f;
+  double f_const, omega, tol;
+  int max_iter;
+  int buf_nodes, slots;
+  double* save;                    // csize * buf_nodes: the field at the start of a batch
+  unsigned long long budget_ns;
+};
+
+// A Gauss-Seidel / SOR solve in the reference's lexicographic order.
+//
+// A sweep visits hyperplanes d = i + j (+ k) in order; a node reads
+// hyperplane d - 1 of this sweep and d + 1 of the one before. So sweep s can
+// work on hyperplane d at step 2 s + d: everything it reads was written one
+// step earlier, and all sweeps in flight work at once. In steady state a
+// step updates every node of one parity, and a sweep costs two steps instead
+// of one barrier per hyperplane; every value is the one of the sequential
+// order.
+//
+// The stopping test needs max|du| of each sweep over steps that overlap with
+// the following sweeps'. A batch of sweeps runs to its end with one flag
+// per sweep ("some |du| >= tol"). When a sweep of the batch passes, the field
+// at the start of the batch is restored and the sweeps before that one are run
+// again; the last sweep always runs alone, with its maximum (the
+// reported delta) and, in 2D, without the closures that the reference
+// applies before a sweep only. Batches grow from 64 to kLexSweeps.
+//
+// Bound by latency, one barrier and a dependent chain per step: 97x65 with
+// Robin and Neumann faces, tol 1e-6, 483 -> 16.5 ms against one barrier per
+// hyperplane in one block (k_gs_lex_block).
+template <int D, class Coef, bool NL>
+__global__ void __launch_bounds__(kClusterThreads + 32) k_cluster_lex(GridDev g, Coef cf, ClusterLexArgs a, NonlinDev nl,
+                                                             double* __restrict__ u, Ctl* ctl) {
+  extern __shared__ double sm[];
+  __shared__ FaceDev face[6];
+  __shared__ unsigned fail[kLexSweeps];   // this CTA's flags; CTA 0 gathers the others' in all_fail
+  __shared__ unsigned all_fail[kLexSweeps];
+  __shared__ double wmax[kClusterThreads / 32];
+  __shared__ double cmax[kClusterMax];
+  __shared__ unsigned long long mbs[2];
+  __shared__ unsigned first_pass, flags;  // flags (CTA 0): 1 degenerate, 2 out of time
+  const unsigned csize = cl_size(), rank = cl_rank();
+  const Slab s = make_slab(g, rank, csize);
+  // all threads copy, the last warp controls the exchange instead of updating nodes
+  const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31;
+  const int nu = nt - 32, nwarps = nu >> 5;
+  const bool control = warp == nwarps;
+  constexpr bool is3 = D == 3;
+  const int half = (g.nx - 1) / 2;              // slots of one parity of a row
+  const int H = is3 ? g.ny - 2 : 1;
+  const int cnt = s.n * H * half;               // slots of one parity
+  double* x = sm;
+  double* sf = x + a.buf_nodes;
+  uint2* tab = reinterpret_cast<uint2*>(sf + a.slots);  // entry and hyperplane
+  double* save = a.save + (size_t)rank * a.buf_nodes;
+  const unsigned long long t0 = globaltimer_ns();
+  if (tid < 6) face[tid] = g.face[tid];
+  if (tid == 0) flags = 0;
+  const unsigned closing = cl_closing(g);
+  ClusterExchange ex;
+  ex.init(s, rank, x, mbs);
+  constexpr bool kConstCoef = std::is_same<Coef, CoefConst>::value;
+  RoundedDiv div;
+  if constexpr (kConstCoef) div.init(cf.c);
+  cl_sync(csize);  // flags of CTA 0 cleared before any CTA sets them
+  const int local = (s.n + 2) * s.L;
+  for (int t = tid; t < local; t += nt) x[t] = u[s.off0 + t];
+  for (int t = tid; t < 2 * cnt; t += nt) {
+    const int p = t >= cnt, r = t - p * cnt, row = r / half, m = r - row * half;
+    const int layer = row / H, q = row - layer * H;
+    const int j = is3 ? 1 + q : s.lo + layer, k = is3 ? s.lo + layer : 0;
+    const int i = 1 + ((p + j + k + 1) & 1) + 2 * m;
+    unsigned e = kClEmpty;
+    if (i <= g.nx - 2) {
+      e = cl_entry(g, s, i, j, k, closing);
+      const int id = s.off0 + (int)((e & kClOffMask) >> 3);
+      sf[t] = a.f ? a.f[id] : a.f_const;
+      if (fabs(cf.template at<double>(g, (long long)id).c) < 1e-12) cl_store_u32(cl_map(&flags, 0), 1u);
+    }
+    tab[t] = make_uint2(e, (unsigned)(i + j + k));
+  }
+  cl_sync(csize);
+  const int nx = g.nx, sxy = is3 ? (int)g.sxy : 0;
+  const int dlo = is3 ? 3 : 2;
+  const int dhi = (g.nx - 2) + (g.ny - 2) + (is3 ? g.nz - 2 : 0);
+  // bytes that the neighbours send in a step of parity p: the nodes of that
+  // parity in the layers before and after this slab
+  unsigned expect[2] = {0u, 0u};
+  for (int side = 0; side < 2; ++side) {
+    if (side == 0 ? !s.has_prev : !s.has_next) continue;
+    const int layer = side == 0 ? s.lo - 1 : s.lo + s.n;
+    for (int p = 0; p < 2; ++p)
+      for (int q = 0; q < H; ++q) {
+        const int i0 = 1 + ((p + layer + (is3 ? 1 + q : 0) + 1) & 1);
+        if (i0 <= g.nx - 2) expect[p] += 8u * (unsigned)((g.nx - 2 - i0) / 2 + 1);
+      }
+  }
+  int step = 0;
+  // the steps of M sweeps of an aligned field. `close`: face closures after
+  // each node; `track`: returns this thread's max|du| (M = 1) instead of
+  // setting the sweeps' flags
+  auto sweeps = [&](int M, bool close, bool track) -> double {
+    double acc = 0.0;
+    for (int tau = dlo; tau <= dhi + 2 * (M - 1); ++tau, ++step) {
+      const int base = (tau & 1) * cnt;
+      const unsigned exp_now = tau & 1 ? expect[1] : expect[0];
+      if (control) {
+        ex.begin(step, exp_now, lane);
+        ex.wait(step);
+      } else {
+        // kClusterNodes nodes of the parity per trip, all computed before
+        // any is stored
+        for (int q0 = tid; q0 < cnt; q0 += kClusterNodes * nu) {
+          uint2 e[kClusterNodes];
+          double rhs[kClusterNodes], old_u[kClusterNodes], upd[kClusterNodes], center[kClusterNodes];
+#pragma unroll
+          for (int m = 0; m < kClusterNodes; ++m) {
+            const int q = base + min(q0 + m * nu, cnt - 1);
+            e[m] = tab[q];
+            // an empty slot reads its row's neighbourhood and is not stored
+            const unsigned off = e[m].x == kClEmpty ? 8u * (unsigned)(s.L + (is3 ? nx : 0) + 1) : e[m].x & kClOffMask;
+            const Stencil<double> st = cf.template at<double, D>(g, (long long)s.off0 + (off >> 3));
+            const double* c = reinterpret_cast<const double*>(reinterpret_cast<const char*>(x) + off);
+            old_u[m] = c[0];
+            const double zp = is3 ? c[sxy] : 0.0, zm = is3 ? c[-sxy] : 0.0;
+            const double lap = nb_sum<double>(st, c[1], c[-1], c[nx], c[-nx], zp, zm, D);
+            const double fv = sf[q];
+            rhs[m] = -(NL ? __dadd_rn(fv, nl_eval(nl, old_u[m])) : fv) - lap;
+            center[m] = st.c;
+          }
+          if constexpr (kConstCoef) {
+            bool fast = div.safe;
+#pragma unroll
+            for (int m = 0; m < kClusterNodes; ++m) {
+              fast = fast && (e[m].x == kClEmpty || div.in_range(rhs[m]));
+              upd[m] = div.fast(rhs[m]);
+            }
+            if (!fast)
+#pragma unroll
+              for (int m = 0; m < kClusterNodes; ++m) upd[m] = __ddiv_rn(rhs[m], div.b);
+          } else {
+#pragma unroll
+            for (int m = 0; m < kClusterNodes; ++m) upd[m] = __ddiv_rn(rhs[m], center[m]);
+          }
+#pragma unroll
+          for (int m = 0; m < kClusterNodes; ++m) {
+            if (q0 + m * nu >= cnt || e[m].x == kClEmpty) continue;
+            const unsigned s2 = (unsigned)(tau - (int)e[m].y);  // twice the sweep of the node
+            const bool active = s2 < (unsigned)(2 * M);
+            double v = old_u[m];
+            if (active) {
+              v = (1.0 - a.omega) * old_u[m] + a.omega * upd[m];
+              *reinterpret_cast<double*>(reinterpret_cast<char*>(x) + (e[m].x & kClOffMask)) = v;
+              const double du = fabs(v - old_u[m]);
+              if (track) {
+                if (du > acc) acc = du;
+              } else if (du >= a.tol) {
+                fail[s2 >> 1] = 1u;
+              }
+            }
+            if (e[m].x >> kClFaceShift) {
+              const unsigned faces = (e[m].x >> kClFaceShift) & 63u;
+              if (active && close && faces) cl_close(g, face, s, x, (int)((e[m].x & kClOffMask) >> 3), faces, v);
+              // nodes outside the sweeps' range are sent as they are: the
+              // neighbours count every node of the parity
+              ex.push(step, e[m].x, 0u, v);
+            }
+          }
+        }
+      }
+      __syncthreads();
+    }
+    return acc;
+  };
+  auto store_own = [&]() {
+    for (int t = tid; t < local; t += nt) {
+      const int layer = t / s.L;
+      if (!((layer == 0 && s.has_prev) || (layer == s.n + 1 && s.has_next))) u[s.off0 + t] = x[t];
+    }
+  };
+  enum { kBatch, kRerun, kLast } phase = kBatch;
+  int done = 0, status = PDEB200_ERR_NOT_CONVERGED, batch = 64, M = 0;
+  double delta = 0.0;
+  const bool degenerate = cl_load_u32(cl_map(&flags, 0)) != 0;
+  if (degenerate) {
+    status = PDEB200_ERR_DEGENERATE;
+    done = 1;
+  }
+  while (!degenerate) {
+    if (phase == kBatch) {
+      M = min(batch, a.max_iter - 1 - done);  // the last allowed sweep runs alone
+      if (M <= 0) phase = kLast;
+    }
+    if (phase == kBatch) {
+      for (int t = tid; t < local; t += nt) save[t] = x[t];
+      for (int t = tid; t < M; t += nt) {
+        fail[t] = 0.0 < a.tol ? 0u : 1u;  // max|du| >= 0 never passes a zero tolerance
+        all_fail[t] = 0u;
+      }
+      if (tid == 0) first_pass = (unsigned)M;
+      cl_sync(csize);
+    } else if (phase == kLast) {
+      M = 1;
+      if constexpr (!is3) {
+        // the closures before the last sweep, edges and corners included: in
+        // 2D the reference leaves the boundary like this
+        store_own();
+        __threadfence();
+        cl_sync(csize);
+        if (rank == 0) block_fill_boundary(g, u, false);
+        __threadfence();
+        cl_sync(csize);
+        for (int t = tid; t < local; t += nt) x[t] = __ldcg(u + s.off0 + t);
+        cl_sync(csize);
+      }
+    }
+    double acc = sweeps(M, phase != kLast || is3, phase == kLast);
+    if (phase == kBatch) {
+      for (int t = tid; t < M; t += nt)
+        if (fail[t]) cl_store_u32(cl_map(&all_fail[t], 0), 1u);
+      if (control && lane == 0 && (ex.dead || (rank == 0 && globaltimer_ns() - t0 > a.budget_ns)))
+        cl_store_u32(cl_map(&flags, 0), 2u);
+      cl_sync(csize);
+      for (int t = tid; t < M; t += nt)
+        if (!cl_load_u32(cl_map(&all_fail[t], 0))) atomicMin(&first_pass, (unsigned)t);
+      const bool late = (cl_load_u32(cl_map(&flags, 0)) & 2u) != 0;
+      cl_sync(csize);
+      const int pass = (int)first_pass;
+      if (pass < M) {
+        for (int t = tid; t < local; t += nt) x[t] = save[t];
+        cl_sync(csize);
+        M = pass;
+        phase = pass > 0 ? kRerun : kLast;
+      } else {
+        done += M;
+        batch = min(2 * batch, kLexSweeps);
+        if (late) {
+          status = PDEB200_ERR_TIMEOUT;
+          break;
+        }
+      }
+    } else if (phase == kRerun) {
+      done += M;
+      phase = kLast;
+    } else {
+      acc = warp_max_nonneg(acc);
+      if (lane == 0 && !control) wmax[warp] = acc;
+      __syncthreads();
+      if (warp == 0) {
+        acc = warp_max_nonneg(lane < nwarps ? wmax[lane] : 0.0);
+        if (lane < (int)csize) cl_store(cl_map(&cmax[rank], lane), acc);
+      }
+      cl_sync(csize);
+      for (unsigned c = 0; c < csize; ++c) delta = fmax(delta, cmax[c]);
+      ++done;
+      if (delta < a.tol) status = PDEB200_OK;
+      break;
+    }
+  }
+  store_own();
+  if (control && lane == 0 && ex.dead) cl_store_u32(cl_map(&flags, 0), 2u);
+  cl_sync(csize);
+  if (rank == 0 && tid == 0) {
+    if (flags & 2u) status = PDEB200_ERR_TIMEOUT;
+    ctl->iter = done;
+    ctl->delta = delta;
+    ctl->status = status;
+    ctl->done = 1;
+  }
+  cl_sync(csize);  // no CTA leaves while another may still access its shared memory
+}
+
 // Multi-block form: one launch per hyperplane; max|du| through an atomic max
 // on the (non-negative) double's bit pattern in ctl->aux[0].
 template <class Coef>
@@ -232,8 +509,28 @@ pdeb200_status gauss_seidel(Context* ctx, DevProblem& P, const Coef& cf, const p
   const long long interior = (long long)(g.nx - 2) * (g.ny - 2) * (g.dim == 3 ? g.nz - 2 : 1);
   if (o->gs_ordering == PDEB200_ORDER_REDBLACK)
     throw StatusFailure{PDEB200_ERR_UNSUPPORTED, "red-black ordering is offered through the MG forms"};
+  const unsigned long long budget = 60ULL * 1000000000ULL;  // device-time guard of the single-launch forms: 60 s
+  const ClusterShape cs = cluster_shape(g, 512);
+  const size_t lex_smem = sizeof(double) * (size_t)cs.buf_nodes + (sizeof(double) + sizeof(uint2)) * (size_t)cs.slots;
+  // grids whose slabs fit in the shared memory of a cluster (about 160k nodes
+  // in 2D): 97x65 SOR 483 -> 16.5 ms, and no grid is faster in the one-block form
+  if (cs.csize > 0 && lex_smem <= kClusterDynSmem) {
+    Buf save(sizeof(double) * (size_t)cs.buf_nodes * cs.csize, ctx->stream);
+    ClusterLexArgs a{P.f, P.f_const, omega, o->tol, max_iter, cs.buf_nodes, cs.slots, save.as<double>(), budget};
+    auto kern = g.dim == 3 ? (P.nl.n ? k_cluster_lex<3, Coef, true> : k_cluster_lex<3, Coef, false>)
+                           : (P.nl.n ? k_cluster_lex<2, Coef, true> : k_cluster_lex<2, Coef, false>);
+    launch_cluster(ctx, cs, lex_smem, kern, g, cf, a, P.nl, d_out, ctx->d_ctl);
+    ctx->count();
+    if (g.dim == 3) fill_boundary(ctx, g, d_out, nullptr);
+    const Ctl& c = ctl_poll(ctx);
+    if (rep) {
+      rep->iterations = c.iter;
+      rep->last_delta = c.delta;
+      rep->converged = c.status == PDEB200_OK;
+    }
+    return (pdeb200_status)c.status;
+  }
   if (interior <= (1LL << 18)) {
-    const unsigned long long budget = 60ULL * 1000000000ULL;  // device-time guard: 60 s
     k_gs_lex_block<Coef><<<1, 1024, 0, ctx->stream>>>(g, cf, P.f, P.f_const, P.nl, d_out, omega, o->tol, max_iter,
                                                       budget,
                                                       ctx->d_ctl);

@@ -22,14 +22,46 @@ pdeb200_status jacobi(Context* ctx, DevProblem& P, const Coef& cf, const pdeb200
                       pdeb200_report* rep) {
   const GridDev& g = P.g;
   const int max_iter = o->max_iter > 1 ? o->max_iter : 1;
-  Buf other(sizeof(double) * g.n, ctx->stream);
   Buf degen(sizeof(int), ctx->stream);
   PDEB_CUDA(cudaMemsetAsync(degen.as<int>(), 0, sizeof(int), ctx->stream));
-  double* buf[2] = {d_out, other.as<double>()};
-  PDEB_CUDA(cudaMemsetAsync(buf[0], 0, sizeof(double) * g.n, ctx->stream));
-  PDEB_CUDA(cudaMemsetAsync(buf[1], 0, sizeof(double) * g.n, ctx->stream));
+  PDEB_CUDA(cudaMemsetAsync(d_out, 0, sizeof(double) * g.n, ctx->stream));
   ctl_init(ctx, max_iter, o->tol, 0.0);
-  fill_boundary(ctx, g, buf[0], ctx->d_ctl);
+  fill_boundary(ctx, g, d_out, ctx->d_ctl);
+  // grids whose slabs fit in the shared memory of a cluster (about 120k nodes
+  // in 2D): whole runs of sweeps in one launch,
+  // 129x129 0.90 against 7.5 us per sweep as launches
+  const ClusterShape cs = cluster_shape(g, 1024);
+  const size_t smem = (2 * sizeof(double)) * (size_t)cs.buf_nodes +
+                      (sizeof(unsigned) + sizeof(double)) * (size_t)cs.cnt_max;
+  if (cs.csize > 0 && smem <= kClusterDynSmem) {
+    constexpr int kSweepsPerLaunch = 2048;  // the host polls and sees a cancel between launches
+    ClusterSweepArgs a{P.f, P.f_const, o->tol, max_iter, 0.0, 0.0, 0, cs.buf_nodes, cs.cnt_max};
+    auto kern = g.dim == 3 ? (P.nl.n ? k_cluster_sweep<3, Coef, false, true> : k_cluster_sweep<3, Coef, false, false>)
+                           : (P.nl.n ? k_cluster_sweep<2, Coef, false, true> : k_cluster_sweep<2, Coef, false, false>);
+    auto run = [&](int q) {
+      a.steps = std::min(kSweepsPerLaunch, max_iter - q * kSweepsPerLaunch);
+      launch_cluster(ctx, cs, smem, kern, g, cf, a, P.nl, d_out, ctx->d_ctl, degen.as<int>());
+      ctx->count();
+    };
+    pdeb200_options po = *o;
+    po.check_interval = 1;
+    const pdeb200_status st = drive(ctx, &po, (max_iter + kSweepsPerLaunch - 1) / kSweepsPerLaunch, run, true);
+    fill_boundary(ctx, g, d_out, nullptr);  // edges and corners
+    const Ctl c = *ctx->h_ctl;
+    int dg = 0;
+    PDEB_CUDA(cudaMemcpyAsync(&dg, degen.as<int>(), sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    PDEB_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (dg) return PDEB200_ERR_DEGENERATE;
+    if (rep) {
+      rep->iterations = c.iter;
+      rep->last_delta = c.delta;
+      rep->converged = st == PDEB200_OK;
+    }
+    return st;
+  }
+  Buf other(sizeof(double) * g.n, ctx->stream);
+  double* buf[2] = {d_out, other.as<double>()};
+  PDEB_CUDA(cudaMemsetAsync(buf[1], 0, sizeof(double) * g.n, ctx->stream));
   const dim3 grid = stencil_grid(g), block = stencil_block();
   auto iterate = [&](int t) {
     double* src = buf[t & 1];
