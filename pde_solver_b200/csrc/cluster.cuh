@@ -24,6 +24,7 @@ constexpr int kClusterMax = 16;      // opt-in cluster size (8 is the portable l
 constexpr int kClusterThreads = 512;  // that update nodes; one more warp controls
 constexpr int kClusterNodes = 2;     // nodes of a thread in flight at once
 constexpr size_t kClusterSmem = 227 * 1024;
+constexpr size_t kClusterDynSmem = kClusterSmem - 10 * 1024;  // the kernels' static shared memory stays below 10 KB
 
 __device__ __forceinline__ unsigned cl_rank() {
   unsigned r;

@@ -271,24 +271,22 @@ inline void launch_dep(const Context* ctx, dim3 grid, dim3 block, size_t smem, v
   PDEB_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
 }
 
-// Launch of a cluster kernel (cluster.cuh): one cluster of cs.csize CTAs. The
+// Launch of a cluster kernel (cluster.cuh): one cluster of csize CTAs. The
 // attributes are the same constants for every launch of a kernel, so threads
 // that launch it at once do not disturb each other.
-constexpr size_t kClusterDynSmem = kClusterSmem - 10 * 1024;  // the kernels' static shared memory stays below 10 KB
-
 template <typename... KArgs, typename... Args>
-inline void launch_cluster(const Context* ctx, const ClusterShape& cs, size_t smem, void (*kern)(KArgs...),
+inline void launch_cluster(const Context* ctx, int csize, int threads, size_t smem, void (*kern)(KArgs...),
                            Args&&... args) {
   PDEB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterDynSmem));
   PDEB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cs.csize);
-  cfg.blockDim = dim3(cs.threads);
+  cfg.gridDim = dim3(csize);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = ctx->stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = cs.csize;
+  attr[0].val.clusterDim.x = csize;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;

@@ -3,6 +3,7 @@
 #include <cstring>
 #include <vector>
 
+#include "cluster_cg.cuh"
 #include "host.h"
 #include "solvers.cuh"
 
@@ -78,25 +79,35 @@ pdeb200_status residual_norms_dev(Context* ctx, DevProblem& P, const double* d_g
 
 // -------------------------------------------------------------- time series
 
+// Closure of face F (constant after inlining) for the node next to it, new value v.
+template <int F>
+__device__ __forceinline__ void fe_close(const GridDev& g, double* next, long long id, int i, int j, int k, double v) {
+  const FaceDev& f = g.face[F];
+  if (f.kind == kDirichlet) return;
+  const long long step = F < kBottom ? 1 : (F < kFront ? g.nx : g.sxy);
+  bool ok;
+  const double b = closure_value(f, F & 1, face_loc(g, F, i, j, k), v, &ok);
+  if (ok) next[(F & 1) ? id + step : id - step] = b;
+}
+
 // One forward-Euler step of SolvePDETimeSeries (solver.cpp:1282-1319):
-// interior next = u + dt * SafeDivClamped(-(L u + f + nonlinear(u)), ut, 0);
-// boundary nodes copied (their closures at t+dt follow in k_fill_boundary).
+// interior next = u + dt * SafeDivClamped(-(L u + f + nonlinear(u)), ut, 0),
+// and the Neumann/Robin closures at t+dt, each written by the thread of the
+// node next to the face (Dirichlet values are in both buffers; edges and
+// corners, which no step reads, are filled when a frame is handed out). With
+// the closures as a launch of their own a step of a small grid cost two
+// launches: FENUM
 template <class Coef>
 __global__ void __launch_bounds__(kBx* kBy) k_fe_step(GridDev g, Coef cf, const double* __restrict__ f, double fc,
                                                       NonlinDev nl, double ut, double dt, const double* __restrict__ u,
                                                       double* __restrict__ next) {
-  const int i = blockIdx.x * kBx + threadIdx.x;
-  const int j = blockIdx.y * kBy + threadIdx.y;
-  if (i >= g.nx || j >= g.ny) return;
-  const int chunk = (g.nz + gridDim.z - 1) / gridDim.z;
-  const int k0 = blockIdx.z * chunk, k1 = min(g.nz, k0 + chunk);
+  const int i = 1 + blockIdx.x * kBx + threadIdx.x;
+  const int j = 1 + blockIdx.y * kBy + threadIdx.y;
+  if (i > g.nx - 2 || j > g.ny - 2) return;
+  int k0, k1;
+  column_range(g, k0, k1);
   for (int k = k0; k < k1; ++k) {
     const long long id = ((long long)k * g.ny + j) * g.nx + i;
-    const bool interior = i >= 1 && i <= g.nx - 2 && j >= 1 && j <= g.ny - 2 && (g.dim == 2 || (k >= 1 && k <= g.nz - 2));
-    if (!interior) {
-      next[id] = u[id];
-      continue;
-    }
     const Stencil<double> s = cf.template at<double>(g, id);
     const double zp = g.dim == 3 ? u[id + g.sxy] : 0.0, zm = g.dim == 3 ? u[id - g.sxy] : 0.0;
     const double opv = s.c * u[id] + nb_sum<double>(s, u[id + 1], u[id - 1], u[id + g.nx], u[id - g.nx], zp, zm, g.dim);
@@ -107,7 +118,16 @@ __global__ void __launch_bounds__(kBx* kBy) k_fe_step(GridDev g, Coef cf, const 
       u_t = -rhs / ut;
       if (!isfinite(u_t)) u_t = 0.0;
     }
-    next[id] = u[id] + dt * u_t;
+    const double v = u[id] + dt * u_t;
+    next[id] = v;
+    if (i == 1) fe_close<kLeft>(g, next, id, i, j, k, v);
+    if (i == g.nx - 2) fe_close<kRight>(g, next, id, i, j, k, v);
+    if (j == 1) fe_close<kBottom>(g, next, id, i, j, k, v);
+    if (j == g.ny - 2) fe_close<kTop>(g, next, id, i, j, k, v);
+    if (g.dim == 3) {
+      if (k == 1) fe_close<kFront>(g, next, id, i, j, k, v);
+      if (k == g.nz - 2) fe_close<kBack>(g, next, id, i, j, k, v);
+    }
   }
 }
 
@@ -118,22 +138,38 @@ pdeb200_status time_series_dev(Context* ctx, DevProblem& P, const pdeb200_time_o
   const long long n = g.n;
   const int frames = t->frames > 1 ? t->frames : 1;
   const int stride = t->frame_stride > 0 ? t->frame_stride : 1;
-  Buf other(sizeof(double) * n, ctx->stream);
-  double* buf[2] = {d_out, other.as<double>()};
+  double* buf[2] = {d_out, nullptr};
   if (P.u0)
     PDEB_CUDA(cudaMemcpyAsync(buf[0], P.u0, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
   else
     PDEB_CUDA(cudaMemsetAsync(buf[0], 0, sizeof(double) * n, ctx->stream));
   fill_boundary(ctx, g, buf[0], nullptr);
+  // grids whose slabs fit in the shared memory of a cluster (about 120k nodes
+  // in 2D) run all steps between two frames in one launch: 257x257, 200 steps
+  // with 5 frames 2.14 -> 0.93 ms
+  const ClusterShape cs = cluster_shape(g, 1024);
+  const size_t smem = (2 * sizeof(double)) * (size_t)cs.buf_nodes +
+                      (sizeof(unsigned) + sizeof(double)) * (size_t)cs.cnt_max;
+  const bool clustered = cs.csize > 0 && smem <= kClusterDynSmem;
+  Buf other;
+  if (!clustered) {
+    other = Buf(sizeof(double) * n, ctx->stream);
+    buf[1] = other.as<double>();
+    PDEB_CUDA(cudaMemcpyAsync(buf[1], buf[0], sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
+  } else {
+    PDEB_CUDA(cudaMemsetAsync(&ctx->d_ctl->status, 0, sizeof(int), ctx->stream));  // a lost cluster reports here
+  }
   std::vector<double> host;
   double* pinned = nullptr;
   if (cb && host_frames) PDEB_CUDA(cudaMallocHost(&pinned, sizeof(double) * n));
   int cur = 0;
   pdeb200_status st = PDEB200_OK;
   PDEB_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
-  const dim3 grid = stencil_grid_full(g), block = stencil_block();
-  for (int frame = 0; frame < frames; ++frame) {
-    if (cb && (frame % stride == 0 || frame + 1 == frames)) {
+  const dim3 grid = stencil_grid_auto(g), block = stencil_block();
+  auto shown = [&](int frame) { return frame % stride == 0 || frame + 1 == frames; };
+  for (int frame = 0; frame < frames;) {
+    if (cb && shown(frame)) {
+      if (frame > 0) fill_boundary(ctx, g, buf[cur], nullptr);  // edges and corners
       const double time = t->t_start + frame * t->dt;
       const double* view = buf[cur];
       if (host_frames) {
@@ -146,19 +182,36 @@ pdeb200_status time_series_dev(Context* ctx, DevProblem& P, const pdeb200_time_o
       if (!cb(frame, time, view, user)) break;
     }
     if (frame + 1 >= frames) break;
+    // steps up to the next frame that is handed out (at most kStepsPerLaunch in one launch)
+    constexpr int kStepsPerLaunch = 1024;
+    int steps = 1;
+    if (clustered)
+      while (steps < kStepsPerLaunch && frame + steps + 1 < frames && !(cb && shown(frame + steps))) ++steps;
     with_coef(P, [&](const auto& cf) {
       using Coef = std::decay_t<decltype(cf)>;
-      k_fe_step<Coef><<<grid, block, 0, ctx->stream>>>(g, cf, P.f, P.f_const, P.nl, P.ut, t->dt, buf[cur],
-                                                       buf[cur ^ 1]);
+      if (clustered) {
+        ClusterSweepArgs a{P.f, P.f_const, 0.0, 0, P.ut, t->dt, steps, cs.buf_nodes, cs.cnt_max};
+        auto kern = g.dim == 3 ? (P.nl.n ? k_cluster_sweep<3, Coef, true, true> : k_cluster_sweep<3, Coef, true, false>)
+                               : (P.nl.n ? k_cluster_sweep<2, Coef, true, true> : k_cluster_sweep<2, Coef, true, false>);
+        launch_cluster(ctx, cs.csize, cs.threads, smem, kern, g, cf, a, P.nl, buf[0], ctx->d_ctl, (int*)nullptr);
+      } else {
+        k_fe_step<Coef><<<grid, block, 0, ctx->stream>>>(g, cf, P.f, P.f_const, P.nl, P.ut, t->dt, buf[cur],
+                                                         buf[cur ^ 1]);
+        cur ^= 1;
+      }
     });
     ctx->count();
-    cur ^= 1;
-    fill_boundary(ctx, g, buf[cur], nullptr);
-    if (rep) rep->iterations = frame + 1;
+    frame += steps;
+    if (rep) rep->iterations = frame;
   }
+  fill_boundary(ctx, g, buf[cur], nullptr);
+  if (clustered)
+    PDEB_CUDA(cudaMemcpyAsync(&ctx->h_ctl->status, &ctx->d_ctl->status, sizeof(int), cudaMemcpyDeviceToHost,
+                              ctx->stream));
   PDEB_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
   if (cur == 1) PDEB_CUDA(cudaMemcpyAsync(d_out, buf[1], sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
   PDEB_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (clustered && ctx->h_ctl->status == PDEB200_ERR_TIMEOUT) st = PDEB200_ERR_TIMEOUT;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
   if (rep) {
@@ -415,35 +468,52 @@ pdeb200_status project_dev(Context* ctx, int nx, int ny, int nz, double dx, doub
   PDEB_CUDA(cudaMemcpyAsync(pc, r, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
   k_dot<double, PostProjR0><<<nb, 256, 0, ctx->stream>>>(n, r, r, ctx->slot(0), PostProjR0{C}, nullptr);
   ctx->count(8);
-  auto iterate = [&](int) {
-    if (!g.is3) {
-      // Ap = L p, sum(Ap) -> mean; Ap -= mean with p.Ap -> alpha
-      k_proj_laplace<PostAux><<<nb, 256, 0, ctx->stream>>>(g, pc, ap, 0, 0, ctx->slot(0), PostAux{C, 3}, C);
-      k_sub_mean<PostProjAlpha><<<nb, 256, 0, ctx->stream>>>(n, ap, pc, 3, ctx->slot(0), PostProjAlpha{C, 0}, C, C);
-      ctx->count(2);
-    } else {
-      k_proj_laplace<PostProjAlpha><<<nb, 256, 0, ctx->stream>>>(g, pc, ap, pin, 1, ctx->slot(0),
-                                                                 PostProjAlpha{C, 1}, C);
-      ctx->count();
-    }
-    k_proj_xr<<<nb, 256, 0, ctx->stream>>>(n, dp, r, pc, ap, ctx->slot(0), PostProjRR{C}, C);
-    k_cg_p<double><<<nb, 256, 0, ctx->stream>>>(n, pc, r, C, 0);
-    ctx->count(2);
-  };
-  // the iteration is captured once as a CUDA graph and replayed (projection
-  // sizes are launch-bound: 256^2 takes about 24 us per iteration as direct launches)
-  IterGraph graph;
-  const bool graphed = graph.capture(ctx, iterate);
-  auto step = [&](int it) {
-    if (graphed)
-      graph.launch(ctx);
-    else
-      iterate(it);
-  };
   pdeb200_options o{};
-  o.check_interval = 32;
-  pdeb200_status st = drive(ctx, &o, po->max_iter + 1, step, false);
-  const Ctl c = ctl_poll(ctx);
+  pdeb200_status st;
+  const CgShape cs = cg_shape(nx, ny, g.nz);
+  if (cs.csize > 0) {
+    // the loop inside one cluster: 256x256 19.5 -> 4.9 us per iteration,
+    // 500x450 81 -> 39 ms
+    CgProj pj{1.0 / (dx * dx), 1.0 / (dy * dy), g.is3 ? 1.0 / (dz * dz) : 0.0, 0.0, pin};
+    pj.cc = -2.0 * (pj.cx + pj.cy + pj.cz);
+    const ClusterCgArgs a{dp, r, pc, ap, kClusterCgIters, nx, ny, g.nz, 0, n};
+    auto kern = g.is3 ? cluster_cg_kernel<kCgProj3, CoefConst>(cs) : cluster_cg_kernel<kCgProj2, CoefConst>(cs);
+    auto run = [&](int) {
+      launch_cluster(ctx, cs.csize, cs.threads, cs.smem, kern, GridDev{}, CoefConst{}, pj, a, C);
+      ctx->count();
+    };
+    o.check_interval = 1;
+    st = drive(ctx, &o, po->max_iter / kClusterCgIters + 1, run, false);
+  } else {
+    auto iterate = [&](int) {
+      if (!g.is3) {
+        // Ap = L p, sum(Ap) -> mean; Ap -= mean with p.Ap -> alpha
+        k_proj_laplace<PostAux><<<nb, 256, 0, ctx->stream>>>(g, pc, ap, 0, 0, ctx->slot(0), PostAux{C, 3}, C);
+        k_sub_mean<PostProjAlpha><<<nb, 256, 0, ctx->stream>>>(n, ap, pc, 3, ctx->slot(0), PostProjAlpha{C, 0}, C, C);
+        ctx->count(2);
+      } else {
+        k_proj_laplace<PostProjAlpha><<<nb, 256, 0, ctx->stream>>>(g, pc, ap, pin, 1, ctx->slot(0),
+                                                                   PostProjAlpha{C, 1}, C);
+        ctx->count();
+      }
+      k_proj_xr<<<nb, 256, 0, ctx->stream>>>(n, dp, r, pc, ap, ctx->slot(0), PostProjRR{C}, C);
+      k_cg_p<double><<<nb, 256, 0, ctx->stream>>>(n, pc, r, C, 0);
+      ctx->count(2);
+    };
+    // the iteration is captured once as a CUDA graph and replayed (projection
+    // sizes are launch-bound: 256^2 takes about 24 us per iteration as direct launches)
+    IterGraph graph;
+    const bool graphed = graph.capture(ctx, iterate);
+    auto step = [&](int it) {
+      if (graphed)
+        graph.launch(ctx);
+      else
+        iterate(it);
+    };
+    o.check_interval = 32;
+    st = drive(ctx, &o, po->max_iter + 1, step, false);
+  }
+  const Ctl c = *ctx->h_ctl;
   const bool zero_start = c.aux[4] != 0.0;
   const bool breakdown = c.aux[7] != 0.0;
   bool ok;

@@ -519,7 +519,7 @@ pdeb200_status gauss_seidel(Context* ctx, DevProblem& P, const Coef& cf, const p
     ClusterLexArgs a{P.f, P.f_const, omega, o->tol, max_iter, cs.buf_nodes, cs.slots, save.as<double>(), budget};
     auto kern = g.dim == 3 ? (P.nl.n ? k_cluster_lex<3, Coef, true> : k_cluster_lex<3, Coef, false>)
                            : (P.nl.n ? k_cluster_lex<2, Coef, true> : k_cluster_lex<2, Coef, false>);
-    launch_cluster(ctx, cs, lex_smem, kern, g, cf, a, P.nl, d_out, ctx->d_ctl);
+    launch_cluster(ctx, cs.csize, cs.threads, lex_smem, kern, g, cf, a, P.nl, d_out, ctx->d_ctl);
     ctx->count();
     if (g.dim == 3) fill_boundary(ctx, g, d_out, nullptr);
     const Ctl& c = ctl_poll(ctx);

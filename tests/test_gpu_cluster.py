@@ -1,5 +1,5 @@
-"""Relaxation runs held in the shared memory of one thread-block cluster
-(Jacobi, lexicographic Gauss-Seidel / SOR) against the oracle, at the sizes
+"""Relaxation runs and heat steps held in the shared memory of one thread-block
+cluster (Jacobi, lexicographic Gauss-Seidel / SOR, forward Euler) against the oracle, at the sizes
 where the slabs, the sweep batches and the launches change: one layer per CTA
 and fewer layers than CTAs, rows of odd and even length, sweep counts around the
 batch and launch sizes, stopping inside a batch.
@@ -97,3 +97,70 @@ def test_cluster_relaxation_constant_f_and_nonlinear(oracle_mod, method):
     check(oracle_mod, p, method=method, max_iter=90, tol=0.0)
     p.nonlinear = [(abi.NL_POWER, 0.4, 2), (abi.NL_SIN, -0.3, 1)]
     check(oracle_mod, p, method=method, max_iter=90, tol=0.0)
+
+
+# the last grid is too large for a cluster: one launch per step
+@pytest.mark.parametrize("dims", [(3, 3, 1), (70, 41, 1), (9, 130, 1), (3, 4, 5), (19, 18, 20), (400, 401, 1)])
+@pytest.mark.parametrize("faces", ["mixed", "arrays"])
+def test_time_series_frames_and_boundaries(oracle_mod, dims, faces):
+    p = make(dims, faces=faces)
+    p.ut = 1.0
+    p.u0 = np.random.Generator(np.random.PCG64(1)).standard_normal(p.n)
+    h = min(1.0 / (d - 1) for d in dims if d > 1)
+    dt = 0.2 * h * h / 2.4
+    seen = {}
+    got, rep = solver.time_series(p, 0.0, dt, 24, on_frame=lambda q, t, u: seen.__setitem__(q, u), frame_stride=7)
+    ref, frames = oracle_mod.rs_time_series(p, 0.0, dt, 24, keep_frames=True)
+    assert rep.iterations == 23 and sorted(seen) == [0, 7, 14, 21, 23]
+    assert rel_l2(got, ref) <= 1e-12
+    for q, u in seen.items():
+        assert rel_l2(u, frames[q]) <= 1e-12
+    assert np.array_equal(got, seen[23])
+
+
+# Krylov loops: the grids are held in shared memory, then with x, r and q in
+# global memory, then by a launch per step. Both sides stop at the same
+# tolerance, so the fields agree to that tolerance times the operator's
+# condition (at most 1e5 here): the 1e-9 bar of the reference CG at tol 1e-12 |b|.
+@pytest.mark.parametrize("dims", [(3, 3, 1), (5, 40, 1), (40, 5, 1), (130, 77, 1), (20, 19, 18), (300, 290, 1),
+                                  (690, 650, 1)])
+@pytest.mark.parametrize("relative", [False, True])
+def test_cluster_cg_sizes(oracle_mod, dims, relative):
+    p = GridProblem(*dims, a=-1.0, b=-2.0, az=-1.0, e=-0.5)
+    x, y, z = p.coords()
+    p.f = np.broadcast_to(np.sin(3.0 * x) * np.cos(2.0 * y) + 0.5 * z, (max(dims[2], 1), dims[1], dims[0])).reshape(-1).copy()
+    bn = np.linalg.norm(p.f)
+    opt = default_options(method=abi.CG, max_iter=6000, tol=1e-12 * (1.0 if relative else bn),
+                          tol_mode=abi.TOL_RELATIVE if relative else abi.TOL_REFERENCE)
+    got, rep = solver.solve(p, opt)
+    st, ref, rrep = oracle_mod.rs_solve(p, default_options(method=abi.CG, max_iter=6000, tol=1e-12 * bn))
+    assert st == 0 and rep.status == abi.OK
+    assert abs(rep.iterations - rrep.iterations) <= 2 + rrep.iterations // 50
+    assert rel_l2(got, ref) <= 1e-9
+
+
+@pytest.mark.parametrize("sweeps", [1, 7])
+def test_cluster_cg_iteration_limit(oracle_mod, sweeps):
+    p = make((41, 38, 1), faces="none")
+    opt = default_options(method=abi.CG, max_iter=sweeps, tol=1e-14)
+    got, rep = solver.solve(p, opt)
+    assert rep.status == abi.ERR_NOT_CONVERGED and rep.iterations == sweeps
+    st, ref, rrep = oracle_mod.rs_solve(p, opt)
+    assert rrep.iterations == sweeps and rel_l2(got, ref) <= 1e-11
+
+
+@pytest.mark.parametrize("dims", [(4, 3, 1), (33, 60, 1), (17, 16, 15), (300, 280, 1), (60, 50, 40)])
+def test_cluster_projection_sizes(oracle_mod, dims):
+    nx, ny, nz = dims
+    rng = np.random.Generator(np.random.PCG64(nx))
+    n = nx * ny * nz
+    u, v = rng.standard_normal(n), rng.standard_normal(n)
+    w = rng.standard_normal(n) if nz > 1 else None
+    h = 1.0 / 40
+    a = (u, v, w, np.zeros(n), nx, ny, nz, h, h, h, 0.01, 20000, 1e-11)
+    ug, vg, wg, pg, rep = solver.project_velocity(*a)
+    _, ur, vr, wr, pr, rrep = oracle_mod.rs_project(*a)
+    assert rep.success == rrep.success
+    assert abs(rep.poisson_iterations - rrep.poisson_iterations) <= 2 + rrep.poisson_iterations // 50
+    for g, r in ((ug, ur), (vg, vr), (pg, pr)) + (((wg, wr),) if nz > 1 else ()):
+        assert rel_l2(g, r) <= 1e-8
