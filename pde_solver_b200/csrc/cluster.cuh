@@ -47,6 +47,15 @@ __device__ __forceinline__ void cl_sync(unsigned csize) {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
 }
+// The end of a kernel: no CTA leaves while another may still access its shared
+// memory. Nothing is published, so the arrival needs no fence.
+__device__ __forceinline__ void cl_leave(unsigned csize) {
+  __syncthreads();
+  if (csize > 1) {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
 // the address of this CTA's shared variable in CTA `rank` of the cluster
 __device__ __forceinline__ unsigned cl_map(const void* p, unsigned rank) {
   unsigned a = (unsigned)__cvta_generic_to_shared(p), r;

@@ -274,24 +274,33 @@ inline void launch_dep(const Context* ctx, dim3 grid, dim3 block, size_t smem, v
 // Launch of a cluster kernel (cluster.cuh): one cluster of csize CTAs. The
 // attributes are the same constants for every launch of a kernel, so threads
 // that launch it at once do not disturb each other.
+// `dep`: with programmatic stream serialization as in launch_dep.
 template <typename... KArgs, typename... Args>
-inline void launch_cluster(const Context* ctx, int csize, int threads, size_t smem, void (*kern)(KArgs...),
-                           Args&&... args) {
-  PDEB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterDynSmem));
+inline void launch_cluster_ex(const Context* ctx, bool dep, size_t max_smem, int csize, int threads, size_t smem,
+                              void (*kern)(KArgs...), Args&&... args) {
+  PDEB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
   PDEB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(csize);
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = ctx->stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = csize;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = dep && ctx->pdl ? 2 : 1;
   PDEB_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...));
+}
+
+template <typename... KArgs, typename... Args>
+inline void launch_cluster(const Context* ctx, int csize, int threads, size_t smem, void (*kern)(KArgs...),
+                           Args&&... args) {
+  launch_cluster_ex(ctx, false, kClusterDynSmem, csize, threads, smem, kern, std::forward<Args>(args)...);
 }
 
 // Dispatch on the coefficient form of a DevProblem: fn(coef) with the concrete type.

@@ -10,6 +10,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "cluster_vcycle.cuh"
 #include "host.h"
 #include "march.cuh"
 #include "sweep.cuh"
@@ -542,6 +543,104 @@ struct Hierarchy {
   int tail_l0 = -1;
   TailLevel<Coef, T>* d_tail = nullptr;
 
+  // Levels from cv_l0 down run inside one cluster (k_cluster_vcycle): the
+  // first level whose arrays, with those of the levels below, fit in the
+  // shared memory of its CTAs (about 33^3 in FP64, 45k nodes in 2D). Not
+  // used when a coarse Neumann/Robin face has per-node closure factors (the
+  // transfer tables are per axis) or the coarsest level has more than
+  // kCvMaxCoarse interior nodes; the single-block tail serves those.
+  int cv_l0 = -1;
+  int cv_csize = 1, cv_coarse = 0;
+  CvLayout cv_layout_;
+  unsigned char* d_cv_image = nullptr;
+  double* d_map = nullptr;
+
+  void build_cluster(Context* ctx) {
+    cv_l0 = -1;
+    const int n = (int)levels.size();
+    const GridDev& gc = levels.back().g;
+    cv_coarse = (int)interior_dofs(gc);
+    if (interior_dofs(gc) > kCvMaxCoarse) return;
+    int first = std::max(0, n - kCvMaxLevels);
+    for (int l = n - 1; l >= 1; --l) {
+      ExtCoef e;
+      if (!ext_coef(levels[l].g, &e)) {
+        first = std::max(first, l);
+        break;
+      }
+    }
+    for (int l = first; l < n; ++l) {
+      if (interior_dofs(levels[l].g) > 1e6) continue;
+      std::vector<CvLevel<Coef, T>> cv(n - l);
+      std::vector<GridDev> gs;
+      for (int m = l; m < n; ++m) gs.push_back(levels[m].g);
+      std::vector<CvGeo> geo(n - l);
+      // levels of up to 512 nodes are faster on one CTA (no exchange), if the memory allows it
+      int csize = 1;
+      CvLayout lay;
+      bool fits = false;
+      for (int single : {512, 64}) {
+        csize = interior_dofs(levels[l].g) > single ? kClusterMax : 1;
+        lay = cv_layout<T>(gs.data(), n - l, csize, single, geo.data());
+        fits = lay.total <= kCvSmem;
+        if (fits) break;
+      }
+      if (!fits) continue;
+      // transfer tables of the pairs (m - 1, m)
+      std::vector<RestrictTap> rt;
+      std::vector<ProlongTap> pt;
+      std::vector<size_t> roff, poff;
+      for (int m = l + 1; m < n; ++m) {
+        const GridDev &f = levels[m - 1].g, &c = levels[m].g;
+        ExtCoef e;
+        ext_coef(c, &e);
+        const int nf[3] = {f.nx, f.ny, f.nz}, nn[3] = {c.nx, c.ny, c.nz};
+        for (int a = 0; a < 3; ++a) {
+          roff.push_back(rt.size());
+          poff.push_back(pt.size());
+          if (a == 2 && f.dim != 3) continue;
+          for (int I = 0; I < nn[a]; ++I) rt.push_back(restrict_tap(I, nf[a], nn[a], e.lo[a], e.hi[a]));
+          for (int i = 0; i < nf[a]; ++i) pt.push_back(prolong_tap(i, nf[a], nn[a], e.lo[a], e.hi[a]));
+        }
+      }
+      const size_t rb = sizeof(RestrictTap) * rt.size(), pb = sizeof(ProlongTap) * pt.size();
+      const size_t lb = sizeof(CvLevel<Coef, T>) * cv.size();
+      owned.emplace_back(lb + rb + pb + sizeof(double) * cv_coarse * cv_coarse + 64, ctx->stream);
+      char* d = owned.back().template as<char>();
+      RestrictTap* drt = reinterpret_cast<RestrictTap*>(d + (lb + 15) / 16 * 16);
+      ProlongTap* dpt = reinterpret_cast<ProlongTap*>(drt + rt.size());
+      d_map = reinterpret_cast<double*>(dpt + pt.size());
+      for (int m = l; m < n; ++m) {
+        ExtCoef e;
+        ext_coef(levels[m].g, &e);
+        cv[m - l].g = levels[m].g;
+        cv[m - l].cf = levels[m].cf;
+        cv[m - l].q = geo[m - l];
+        for (int a = 0; a < 3; ++a) {
+          cv[m - l].q.lo[a] = e.lo[a];
+          cv[m - l].q.hi[a] = e.hi[a];
+          cv[m - l].q.rt[a] = m > l ? drt + roff[3 * (m - l - 1) + a] : nullptr;
+          cv[m - l].q.pt[a] = m + 1 < n ? dpt + poff[3 * (m - l) + a] : nullptr;
+        }
+      }
+      CvLevel<Coef, T>* d_cv = reinterpret_cast<CvLevel<Coef, T>*>(d);
+      owned.emplace_back(lay.image * csize, ctx->stream);
+      d_cv_image = owned.back().template as<unsigned char>();
+      PDEB_CUDA(cudaMemcpyAsync(d_cv, cv.data(), lb, cudaMemcpyHostToDevice, ctx->stream));
+      if (rb) PDEB_CUDA(cudaMemcpyAsync(drt, rt.data(), rb, cudaMemcpyHostToDevice, ctx->stream));
+      if (pb) PDEB_CUDA(cudaMemcpyAsync(dpt, pt.data(), pb, cudaMemcpyHostToDevice, ctx->stream));
+      k_coarse_map<Coef><<<cv_coarse, kCvMaxCoarse, 0, ctx->stream>>>(levels.back().g, levels.back().cf, coarse_iters,
+                                                                      d_map);
+      k_cv_image<Coef, T><<<dim3(csize, n - l), 256, 0, ctx->stream>>>(d_cv, n - l, lay.image, d_cv_image);
+      ctx->count(2);
+      PDEB_CUDA(cudaStreamSynchronize(ctx->stream));
+      cv_csize = csize;
+      cv_layout_ = lay;
+      cv_l0 = l;
+      return;
+    }
+  }
+
   bool coarse_in_smem(const Level& L) const {
     const long long interior = (long long)(L.g.nx - 2) * (L.g.ny - 2) * (L.g.dim == 3 ? L.g.nz - 2 : 1);
     return L.g.n <= kCoarseMaxNodes && interior <= kCoarseMaxInterior;
@@ -590,7 +689,9 @@ struct Hierarchy {
     // single-block tail: the first level small enough, with at most
     // kTailMaxLevels levels below it (colour-pass form only)
     tail_l0 = -1;
-    if (!fused && std::getenv("PDEB200_NO_TAIL") == nullptr) {
+    cv_l0 = -1;
+    if (!fused && std::getenv("PDEB200_NO_TAIL") == nullptr) build_cluster(ctx);
+    if (cv_l0 < 0 && !fused && std::getenv("PDEB200_NO_TAIL") == nullptr) {
       for (size_t l = 0; l < levels.size(); ++l)
         if (levels[l].g.n <= kTailMaxNodes && (int)(levels.size() - l) <= kTailMaxLevels) {
           tail_l0 = (int)l;
@@ -628,6 +729,7 @@ struct Hierarchy {
         flips = pre > 0 ? pre - 1 + post : post;
       L.out = (flips & 1) ? L.xb : L.xa;
     }
+    if (cv_l0 >= 0) levels[cv_l0].out = levels[cv_l0].xa;
   }
 
   // `sweeps` red-black sweeps starting from `cur` (or from zero); returns the
@@ -743,6 +845,15 @@ struct Hierarchy {
     Level& L = levels[l];
     const T* b = l == 0 ? rhs0 : L.b;
     const double dofs = interior_dofs(L.g);
+    if (l == cv_l0) {
+      ProfScope ps(ctx, "cluster_vcycle", l, 0.0);
+      launch_cluster_ex(ctx, true, kCvSmem, cv_csize, kCvThreads + 32, cv_layout_.total, k_cluster_vcycle<T>,
+                        (const unsigned char*)d_cv_image, (unsigned)cv_layout_.image,
+                        (unsigned)cv_layout_.total, (int)levels.size() - l, b, L.xa, pre, post, (const double*)d_map,
+                        cv_coarse, const_cast<Ctl*>(ctl));
+      ctx->count();
+      return;
+    }
     if (l == tail_l0) {
       ProfScope ps(ctx, "tail_vcycle", l, 0.0);
       launch_dep(ctx, dim3(1), dim3(kTailThreads), 0, k_tail_vcycle<Coef, T>, (const TailLevel<Coef, T>*)d_tail,
