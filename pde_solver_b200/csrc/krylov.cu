@@ -568,20 +568,9 @@ pdeb200_status mg_bicgstab_core(Context* ctx, HierT& H, const GridDev& g, const 
     k_bi_r<T, PostBiResid><<<nb, 256, 0, ctx->stream>>>(n, r, s, t, ctx->slot(), PostBiResid{C, 1}, C);
     ctx->count(12);
   };
-  // iterations after the first are identical: replay them as a graph
-  IterGraph graph;
-  int graphed = -1;
-  auto step = [&](int it) {
-    if (it == 0) {
-      iterate(0);
-      return;
-    }
-    if (graphed < 0) graphed = graph.capture(ctx, [&](int) { iterate(1); }) ? 1 : 0;
-    if (graphed)
-      graph.launch(ctx);
-    else
-      iterate(it);
-  };
+  // iterations after the first are identical
+  StepGraph graph;
+  auto step = [&](int it) { graph.step(ctx, n, it, iterate, [&](int) { iterate(1); }); };
   pdeb200_status st = drive(ctx, o, max_iter + 1, step, false);
   const Ctl c = ctl_poll(ctx);
   *iters = c.iter;
@@ -680,9 +669,7 @@ __global__ void k_add_scaled(long long n, double* __restrict__ x, const T* __res
 template <class Coef, class HierT, typename T>
 struct MgPcgCore {
   Buf buf;
-  IterGraph graph;
-  int graphed = -1;  // -1: not captured yet
-  bool fused_dot = false;
+  StepGraph graph;
 
   pdeb200_status run(Context* ctx, HierT& H, const GridDev& g, const Coef& cf, const T* b, T* x, int max_iter,
                      double tol, const pdeb200_options* o, int* iters) {
@@ -704,23 +691,20 @@ struct MgPcgCore {
     ctx->count(3);
     const dim3 grid = stencil_grid_auto(g), block = stencil_block();
     auto iterate = [&](int) {
-      k_apply_folded<Coef, T, 1, PostAlpha><<<grid, block, 0, ctx->stream>>>(g, cf, p, q, ctx->slot(), PostAlpha{C}, C);
-      k_cg_xr<T, PostRRRel><<<nb, 256, 0, ctx->stream>>>(n, x, r, p, q, ctx->slot(), PostRRRel{C}, C);
+      launch_dep(ctx, grid, block, 0, k_apply_folded<Coef, T, 1, PostAlpha>, g, cf, (const T*)p, q, ctx->slot(),
+                 PostAlpha{C}, (const Ctl*)C);
+      launch_dep(ctx, dim3(nb), dim3(256), 0, k_cg_xr<T, PostRRRel>, n, x, r, (const T*)p, (const T*)q, ctx->slot(),
+                 PostRRRel{C}, C);
       // beta from r.z summed by the preconditioner's last colour passes when it can
       if (!H.vcycle_dot(ctx, r, C, ctx->slot())) {
-        k_dot<T, PostBeta><<<nb, 256, 0, ctx->stream>>>(n, r, z, ctx->slot(), PostBeta{C}, C);
+        launch_dep(ctx, dim3(nb), dim3(256), 0, k_dot<T, PostBeta>, n, (const T*)r, (const T*)z, ctx->slot(),
+                   PostBeta{C}, (const Ctl*)C);
         ctx->count();
       }
-      k_cg_p<T><<<nb, 256, 0, ctx->stream>>>(n, p, z, C, 0);
+      launch_dep(ctx, dim3(nb), dim3(256), 0, k_cg_p<T>, n, p, (const T*)z, (const Ctl*)C, 0);
       ctx->count(3);
     };
-    if (graphed < 0) graphed = graph.capture(ctx, iterate) ? 1 : 0;
-    auto step = [&](int it) {
-      if (graphed)
-        graph.launch(ctx);
-      else
-        iterate(it);
-    };
+    auto step = [&](int it) { graph.step(ctx, n, it, iterate, iterate); };
     pdeb200_status st = drive(ctx, o, max_iter + 1, step, false);
     const Ctl c = ctl_poll(ctx);
     *iters = c.iter;

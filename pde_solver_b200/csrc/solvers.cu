@@ -192,8 +192,7 @@ pdeb200_status mg_pcg(Context* ctx, DevProblem& P, const Coef& cf, const pdeb200
   build_folded_rhs(ctx, P, cf, bf);
   PDEB_CUDA(cudaMemsetAsync(d_x, 0, sizeof(double) * n, ctx->stream));
   PDEB_CUDA(cudaMemcpyAsync(r, bf, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
-  PDEB_CUDA(cudaMemsetAsync(p, 0, sizeof(double) * n, ctx->stream));
-  PDEB_CUDA(cudaMemsetAsync(q, 0, sizeof(double) * n, ctx->stream));
+  PDEB_CUDA(cudaMemsetAsync(q, 0, sizeof(double) * n, ctx->stream));  // its boundary is never written
   const int nb = vec_blocks(n, ctx);
   k_dot<double, PostBB><<<nb, 256, 0, ctx->stream>>>(n, bf, bf, ctx->slot(), PostBB{ctx->d_ctl}, ctx->d_ctl);
   ctx->count();
@@ -231,14 +230,8 @@ pdeb200_status mg_pcg(Context* ctx, DevProblem& P, const Coef& cf, const pdeb200
     }
     ctx->count(2);
   };
-  IterGraph graph;
-  const bool graphed = graph.capture(ctx, iterate);
-  auto step = [&](int it) {
-    if (graphed)
-      graph.launch(ctx);
-    else
-      iterate(it);
-  };
+  StepGraph graph;
+  auto step = [&](int it) { graph.step(ctx, n, it, iterate, iterate); };
   // |r|^2 <= tol2 on the device (PostRRRel): batches sized by the observed reduction rate
   pdeb200_status st = drive(ctx, o, max_iter + 1, step, false, true);
   const Ctl c = ctl_poll(ctx);

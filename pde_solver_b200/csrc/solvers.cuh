@@ -275,6 +275,35 @@ struct IterGraph {
   }
 };
 
+// The iterations of a multigrid-preconditioned Krylov solve. The first two are
+// launched directly, so the device is busy while the host captures and
+// instantiates the graph that replays the rest (0.3 to 0.5 ms, more than an
+// iteration of a small grid); a solve of one or two iterations never captures.
+// Iterations of at most kDirectLaunches launches stay direct: the host launches
+// one in about 2.3 us, less than their kernels take, and capture,
+// instantiation and destruction (0.5 ms) are not earned back: 257x193 1.72 ->
+// 1.52 ms with one memset for all levels. So do those of grids above
+// kDirectNodes, whose kernels take 5 us and more: 513^3 mixed BiCGStab 85.6 -> 84.3 ms.
+struct StepGraph {
+  static constexpr long long kDirectLaunches = 24;
+  static constexpr long long kDirectNodes = 1LL << 20;
+  IterGraph graph;
+  int state = -1;  // -1 not tried, 0 direct, 1 replay
+  long long launches = 0;
+  // `first`: enqueues iteration `it` directly; `repeat`: the one to replay
+  template <class First, class Repeat>
+  void step(Context* ctx, long long n, int it, First&& first, Repeat&& repeat) {
+    if (state < 0 && it >= 2 && launches > kDirectLaunches && n <= kDirectNodes) state = graph.capture(ctx, repeat) ? 1 : 0;
+    if (state == 1) {
+      graph.launch(ctx);
+      return;
+    }
+    const long long before = ctx->launches;
+    first(it);
+    launches = ctx->launches - before;
+  }
+};
+
 inline void fill_boundary(Context* ctx, const GridDev& g, double* u, const Ctl* ctl, bool dirichlet_last = true) {
   const long long faces = 2LL * g.ny * g.nz + 2LL * g.nx * g.nz + (g.dim == 3 ? 2LL * g.nx * g.ny : 0);
   const int blocks = vec_blocks(faces, ctx);
@@ -531,11 +560,27 @@ struct Hierarchy {
   int pre = 2, post = 2, coarse_iters = 50;
   bool needs_fold = false;  // some face is Neumann/Robin
 
-  T* alloc(Context* ctx, long long n) {
-    owned.emplace_back(sizeof(T) * n, ctx->stream);
+  // The levels' vectors in one zeroed allocation (one memset instead of four
+  // per level); xb only for the single-pass sweep forms, which alone use it.
+  void place_vectors(Context* ctx, bool two_fields) {
+    auto padded = [](long long n) { return (n + 63) / 64 * 64; };
+    long long total = 0;
+    for (size_t l = 0; l < levels.size(); ++l) total += padded(levels[l].g.n) * ((l ? 3 : 2) + (two_fields ? 1 : 0));
+    owned.emplace_back(sizeof(T) * total, ctx->stream);
     T* p = owned.back().template as<T>();
-    PDEB_CUDA(cudaMemsetAsync(p, 0, sizeof(T) * n, ctx->stream));
-    return p;
+    PDEB_CUDA(cudaMemsetAsync(p, 0, sizeof(T) * total, ctx->stream));
+    for (size_t l = 0; l < levels.size(); ++l) {
+      Level& L = levels[l];
+      auto take = [&]() {
+        T* q = p;
+        p += padded(L.g.n);
+        return q;
+      };
+      L.xa = take();
+      L.r = take();
+      L.b = l ? take() : nullptr;
+      L.xb = two_fields ? take() : nullptr;
+    }
   }
 
   // Levels from tail_l0 down run as one single-block launch (k_tail_vcycle).
@@ -658,10 +703,6 @@ struct Hierarchy {
     Level l0;
     l0.g = P.g;
     l0.cf = cf0;
-    l0.xa = alloc(ctx, P.g.n);
-    l0.xb = alloc(ctx, P.g.n);
-    l0.b = nullptr;
-    l0.r = alloc(ctx, P.g.n);
     levels.push_back(l0);
     int stride = 1;
     int nc[3];
@@ -680,12 +721,11 @@ struct Hierarchy {
       const double cdz = gf.dim == 3 ? (hp->zmax - hp->zmin) / (double)(c.g.nz - 1) : 0.0;
       build_faces(ctx, hp, c.g.nx, c.g.ny, c.g.nz, cdx, cdy, cdz, stride, &c.g, &owned);
       c.cf = coarsen_coef(ctx, P, levels.back().cf, gf, c.g, cdx, cdy, cdz, &owned);
-      c.xa = alloc(ctx, c.g.n);
-      c.xb = alloc(ctx, c.g.n);
-      c.b = alloc(ctx, c.g.n);
-      c.r = alloc(ctx, c.g.n);
       levels.push_back(c);
     }
+    const bool sweep_env = std::getenv("PDEB200_STAGED_SWEEP") != nullptr;
+    const bool march_env = std::getenv("PDEB200_MARCH") != nullptr;
+    place_vectors(ctx, fused || sweep_env || march_env);
     // single-block tail: the first level small enough, with at most
     // kTailMaxLevels levels below it (colour-pass form only)
     tail_l0 = -1;
@@ -710,8 +750,6 @@ struct Hierarchy {
     }
     // result buffer of each level after a V-cycle (fixed, so launches can be captured):
     // the first sweep from zero writes xa, every later sweep flips the buffer
-    const bool sweep_env = std::getenv("PDEB200_STAGED_SWEEP") != nullptr;
-    const bool march_env = std::getenv("PDEB200_MARCH") != nullptr;
     for (size_t l = 0; l < levels.size(); ++l) {
       Level& L = levels[l];
       L.single_pass = kSweepCoef && sweep_env && !fused && l + 1 < levels.size() && L.g.dim == 3 &&
