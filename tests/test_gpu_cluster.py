@@ -164,3 +164,32 @@ def test_cluster_projection_sizes(oracle_mod, dims):
     assert abs(rep.poisson_iterations - rrep.poisson_iterations) <= 2 + rrep.poisson_iterations // 50
     for g, r in ((ug, ur), (vg, vr), (pg, pr)) + (((wg, wr),) if nz > 1 else ()):
         assert rel_l2(g, r) <= 1e-8
+
+
+# One and several virtual blocks and rounds; the 3D grid is served by launches. Both sides stop at a true residual of 1e-9 |b|, so the fields differ by
+# at most 2e-9 times the condition number, about (n / 2)^2 in n nodes a side.
+@pytest.mark.parametrize("dims", [(3, 3, 1), (3, 50, 1), (6, 40, 1), (40, 6, 1), (97, 81, 1), (161, 150, 1),
+                                  (20, 19, 18)])
+@pytest.mark.parametrize("coef", ["const", "nodal"])
+@pytest.mark.parametrize("relative", [False, True])
+def test_cluster_bicgstab_sizes(oracle_mod, dims, coef, relative):
+    p = make(dims, coef, faces="none")
+    x, y, z = p.coords()
+    p.f = np.broadcast_to(np.sin(3.0 * x) * np.cos(2.0 * y) + 0.5 * z, (max(dims[2], 1), dims[1], dims[0])).reshape(-1).copy()
+    bn = np.linalg.norm(p.f)
+    opt = default_options(method=abi.BICGSTAB, max_iter=6000, tol=1e-9 * (1.0 if relative else bn),
+                          tol_mode=abi.TOL_RELATIVE if relative else abi.TOL_REFERENCE)
+    got, rep = solver.solve(p, opt)
+    st, ref, _ = oracle_mod.rs_solve(p, default_options(method=abi.BICGSTAB, max_iter=6000, tol=1e-9 * bn))
+    assert st == 0 and rep.status == abi.OK and rep.residual_l2 <= 1.01e-9 * bn
+    assert rel_l2(got, ref) <= 2e-9 * (max(dims) / 2) ** 2
+
+
+@pytest.mark.parametrize("iterations", [1, 2, 9])
+def test_cluster_bicgstab_iteration_limit(oracle_mod, iterations):
+    p = make((41, 38, 1), "nodal", faces="none")
+    opt = default_options(method=abi.BICGSTAB, max_iter=iterations, tol=1e-14)
+    got, rep = solver.solve(p, opt)
+    st, ref, rrep = oracle_mod.rs_solve(p, opt)
+    assert rep.status == abi.ERR_NOT_CONVERGED and rep.iterations == rrep.iterations == iterations
+    assert rel_l2(got, ref) <= 1e-9
