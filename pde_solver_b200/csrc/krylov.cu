@@ -706,7 +706,7 @@ struct MgPcgCore {
     k_dot<T, PostRZ><<<nb, 256, 0, ctx->stream>>>(n, r, z, ctx->slot(), PostRZ{C}, C);
     k_cg_p<T><<<nb, 256, 0, ctx->stream>>>(n, p, z, C, 1);
     ctx->count(3);
-    const dim3 grid = stencil_grid_auto(g), block = stencil_block();
+    const dim3 grid = apply_grid(g), block = stencil_block();
     auto iterate = [&](int) {
       launch_dep(ctx, grid, block, 0, k_apply_folded<Coef, T, 1, PostAlpha>, g, cf, (const T*)p, q, ctx->slot(),
                  PostAlpha{C}, (const Ctl*)C);

@@ -203,7 +203,7 @@ pdeb200_status mg_pcg(Context* ctx, DevProblem& P, const Coef& cf, const pdeb200
   k_dot<double, PostRZ><<<nb, 256, 0, ctx->stream>>>(n, r, z, ctx->slot(), PostRZ{ctx->d_ctl}, ctx->d_ctl);
   k_cg_p<double><<<nb, 256, 0, ctx->stream>>>(n, p, z, ctx->d_ctl, 1);
   ctx->count(2);
-  const dim3 grid = stencil_grid_auto(g), block = stencil_block();
+  const dim3 grid = apply_grid(g), block = stencil_block();
   const double dofs = interior_dofs(g);
   auto iterate = [&](int) {
     {

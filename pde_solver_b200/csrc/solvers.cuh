@@ -463,6 +463,20 @@ inline dim3 prolong_grid(const GridDev& g) {
   return dim3(xy.x, xy.y, (unsigned)chunks);
 }
 
+// launch shape of k_restrict_taps: 32 x 8 interior coarse columns per block; 4
+// coarse planes per thread share plane sums on large levels (into 129^3: 58.3
+// us, against 61.3 with 8 and 76.0 with 16), small levels take one plane per
+// thread (latency rather than bytes)
+inline dim3 restrict_grid(const GridDev& g) {
+  const dim3 xy((g.nx - 2 + kBx - 1) / kBx, (g.ny - 2 + kBy - 1) / kBy, 1);
+  const long long xyb = (long long)xy.x * xy.y;
+  const int kint = g.dim == 3 ? g.nz - 2 : 1, zc = g.n > (1LL << 20) ? 4 : 1;
+  long long chunks = (kint + zc - 1) / zc;
+  if (chunks > kMaxGridBlocks / xyb) chunks = kMaxGridBlocks / xyb;
+  if (chunks < 1) chunks = 1;
+  return dim3(xy.x, xy.y, (unsigned)chunks);
+}
+
 template <typename KT>
 inline void inject_k(Context* ctx, const GridDev& gf, const GridDev& gc, const KT* kf, KT* kc) {
   k_inject<KT><<<vec_blocks(gc.n, ctx), 256, 0, ctx->stream>>>(gf, gc, kf, kc);
@@ -535,6 +549,7 @@ struct Hierarchy {
     T* b;
     T* r;
     T* out;  // buffer holding this level's result after a V-cycle
+    const RestrictTap* rt[3] = {nullptr, nullptr, nullptr};  // restriction onto this level (null: ext factors per node)
     bool single_pass = false;  // sweeps by k_rbgs_sweep (x_in -> x_out) instead of colour passes
     bool march = false;        // sweeps by k_rbgs_march (x_in -> x_out) instead of colour passes
   };
@@ -600,6 +615,30 @@ struct Hierarchy {
   unsigned char* d_cv_image = nullptr;
   double* d_map = nullptr;
 
+  // restriction taps of every level whose closure factors are per face
+  void build_taps(Context* ctx) {
+    std::vector<RestrictTap> rt;
+    std::vector<size_t> off(3 * levels.size(), 0);
+    std::vector<char> on(levels.size(), 0);
+    for (size_t m = 1; m < levels.size(); ++m) {
+      const GridDev &f = levels[m - 1].g, &c = levels[m].g;
+      ExtCoef e;
+      if (!ext_coef(c, &e)) continue;
+      on[m] = 1;
+      const int nf[3] = {f.nx, f.ny, f.nz}, nc[3] = {c.nx, c.ny, c.nz};
+      for (int a = 0; a < f.dim; ++a) {
+        off[3 * m + a] = rt.size();
+        for (int I = 0; I < nc[a]; ++I) rt.push_back(restrict_tap(I, nf[a], nc[a], e.lo[a], e.hi[a]));
+      }
+    }
+    if (rt.empty()) return;
+    owned.emplace_back(sizeof(RestrictTap) * rt.size(), ctx->stream);
+    RestrictTap* d = owned.back().template as<RestrictTap>();
+    PDEB_CUDA(cudaMemcpyAsync(d, rt.data(), sizeof(RestrictTap) * rt.size(), cudaMemcpyHostToDevice, ctx->stream));
+    for (size_t m = 1; m < levels.size(); ++m)
+      for (int a = 0; a < 3; ++a) levels[m].rt[a] = on[m] ? d + off[3 * m + a] : nullptr;
+  }
+
   void build_cluster(Context* ctx) {
     cv_l0 = -1;
     const int n = (int)levels.size();
@@ -632,28 +671,24 @@ struct Hierarchy {
       }
       if (!fits) continue;
       // transfer tables of the pairs (m - 1, m)
-      std::vector<RestrictTap> rt;
       std::vector<ProlongTap> pt;
-      std::vector<size_t> roff, poff;
+      std::vector<size_t> poff;
       for (int m = l + 1; m < n; ++m) {
         const GridDev &f = levels[m - 1].g, &c = levels[m].g;
         ExtCoef e;
         ext_coef(c, &e);
         const int nf[3] = {f.nx, f.ny, f.nz}, nn[3] = {c.nx, c.ny, c.nz};
         for (int a = 0; a < 3; ++a) {
-          roff.push_back(rt.size());
           poff.push_back(pt.size());
           if (a == 2 && f.dim != 3) continue;
-          for (int I = 0; I < nn[a]; ++I) rt.push_back(restrict_tap(I, nf[a], nn[a], e.lo[a], e.hi[a]));
           for (int i = 0; i < nf[a]; ++i) pt.push_back(prolong_tap(i, nf[a], nn[a], e.lo[a], e.hi[a]));
         }
       }
-      const size_t rb = sizeof(RestrictTap) * rt.size(), pb = sizeof(ProlongTap) * pt.size();
+      const size_t pb = sizeof(ProlongTap) * pt.size();
       const size_t lb = sizeof(CvLevel<Coef, T>) * cv.size();
-      owned.emplace_back(lb + rb + pb + sizeof(double) * cv_coarse * cv_coarse + 64, ctx->stream);
+      owned.emplace_back(lb + pb + sizeof(double) * cv_coarse * cv_coarse + 64, ctx->stream);
       char* d = owned.back().template as<char>();
-      RestrictTap* drt = reinterpret_cast<RestrictTap*>(d + (lb + 15) / 16 * 16);
-      ProlongTap* dpt = reinterpret_cast<ProlongTap*>(drt + rt.size());
+      ProlongTap* dpt = reinterpret_cast<ProlongTap*>(d + (lb + 15) / 16 * 16);
       d_map = reinterpret_cast<double*>(dpt + pt.size());
       for (int m = l; m < n; ++m) {
         ExtCoef e;
@@ -664,7 +699,7 @@ struct Hierarchy {
         for (int a = 0; a < 3; ++a) {
           cv[m - l].q.lo[a] = e.lo[a];
           cv[m - l].q.hi[a] = e.hi[a];
-          cv[m - l].q.rt[a] = m > l ? drt + roff[3 * (m - l - 1) + a] : nullptr;
+          cv[m - l].q.rt[a] = m > l ? levels[m].rt[a] : nullptr;
           cv[m - l].q.pt[a] = m + 1 < n ? dpt + poff[3 * (m - l) + a] : nullptr;
         }
       }
@@ -672,7 +707,6 @@ struct Hierarchy {
       owned.emplace_back(lay.image * csize, ctx->stream);
       d_cv_image = owned.back().template as<unsigned char>();
       PDEB_CUDA(cudaMemcpyAsync(d_cv, cv.data(), lb, cudaMemcpyHostToDevice, ctx->stream));
-      if (rb) PDEB_CUDA(cudaMemcpyAsync(drt, rt.data(), rb, cudaMemcpyHostToDevice, ctx->stream));
       if (pb) PDEB_CUDA(cudaMemcpyAsync(dpt, pt.data(), pb, cudaMemcpyHostToDevice, ctx->stream));
       k_coarse_map<Coef><<<cv_coarse, kCvMaxCoarse, 0, ctx->stream>>>(levels.back().g, levels.back().cf, coarse_iters,
                                                                       d_map);
@@ -726,6 +760,7 @@ struct Hierarchy {
     const bool sweep_env = std::getenv("PDEB200_STAGED_SWEEP") != nullptr;
     const bool march_env = std::getenv("PDEB200_MARCH") != nullptr;
     place_vectors(ctx, fused || sweep_env || march_env);
+    build_taps(ctx);
     // single-block tail: the first level small enough, with at most
     // kTailMaxLevels levels below it (colour-pass form only)
     tail_l0 = -1;
@@ -929,7 +964,11 @@ struct Hierarchy {
     Level& C = levels[l + 1];
     {
       ProfScope ps(ctx, "restrict", l, dofs * sizeof(T) * (1.0 + 1.0 / (L.g.dim == 3 ? 8.0 : 4.0)));
-      if (z_nested(L.g, C.g))
+      if (C.rt[0])
+        launch_dep(ctx, restrict_grid(C.g), stencil_block(), 0, k_restrict_taps<T>, level_geo(L.g), level_geo(C.g),
+                   C.rt[0], C.rt[1], C.rt[2], 2 * C.g.nx - 1 == L.g.nx && 2 * C.g.ny - 1 == L.g.ny ? 1 : 0,
+                   L.g.dim == 3 && 2 * C.g.nz - 1 == L.g.nz ? 1 : 0, (const T*)L.r, C.b, ctl);
+      else if (z_nested(L.g, C.g))
         // 4 coarse planes per thread share plane sums on large levels (into
         // 129^3: 58.3 us, against 61.3 with 8 and 76.0 with 16); small levels
         // take one plane per thread (latency rather than bytes). The result
@@ -941,7 +980,7 @@ struct Hierarchy {
         launch_dep(ctx, stencil_grid_full(C.g, 1), stencil_block(), 0, k_restrict_fw<T, T>, L.g, C.g, (const T*)L.r,
                    C.b, ctl);
     }
-    if (needs_fold) {
+    if (needs_fold && !C.rt[0]) {
       ProfScope ps(ctx, "restrict_fold", l, 0.0);
       const FoldLayers lay = fold_layers(C.g);
       const int blocks = (int)std::max<long long>(1, std::min<long long>((lay.start[6] + 255) / 256, 148LL * 16));
