@@ -9,7 +9,9 @@
 #include <cstdlib>
 #include <cstring>
 #include <fstream>
+#include <map>
 #include <memory>
+#include <tuple>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -51,6 +53,10 @@ struct BatchPlan {
   double *f64 = nullptr, *b64 = nullptr, *x64 = nullptr;
   std::vector<Buf> owned;          // face arrays of coarse levels
   Buf d_levels, d_mem, d_active;
+  std::vector<int> tail_lev;       // member -> first level of its tail, or -1
+  std::vector<int> tail_rec;       // member -> tail record
+  Buf d_taps, d_tails, d_tail_images;
+  unsigned tail_smem = 0;          // largest tail
   std::unique_ptr<Sched> full;  // tiles of every member (set by build_schedule)
   int* h_active = nullptr;
   BMember* h_mem = nullptr;
@@ -69,7 +75,8 @@ struct BatchPlan {
 // reduction partials sized for its level-0 tiles, each member's level-0 tile
 // range and the captured cycle.
 struct Sched {
-  Buf tiles, partials;
+  Buf tiles, partials, tails;
+  int ntails = 0;
   std::vector<long long> off, cnt;
   std::vector<int> tile0, ntiles;  // per member; ntiles 0 when absent
   int lmax = 0;
@@ -99,6 +106,9 @@ BatchPlan::~BatchPlan() {
     a64.reset();
     a32.reset();
     akh.reset();
+    d_tails.reset();
+    d_taps.reset();
+    d_tail_images.reset();
     d_levels.reset();
     d_mem.reset();
     d_active.reset();
@@ -118,7 +128,8 @@ long long interior_nodes(const GridDev& g) {
 }
 
 // Tiles of one level of one member (interior nodes only).
-void make_tiles(const GridDev& g, bool coarse, const BatchParams& p, int lev, int member, std::vector<BTile>* out) {
+void make_tiles(const GridDev& g, bool coarse, bool tail, const BatchParams& p, int lev, int member,
+                std::vector<BTile>* out) {
   const int ni = g.nx - 2, nj = g.ny - 2;
   const int kb = g.dim == 3 ? 1 : 0, ke = g.dim == 3 ? g.nz - 1 : 1;
   auto tile = [&](int x0, int y0, int w, int h, int z0, int z1, int coarse_flag) {
@@ -136,6 +147,7 @@ void make_tiles(const GridDev& g, bool coarse, const BatchParams& p, int lev, in
     while ((1 << lw) < w) ++lw;
     t.lw = (unsigned char)lw;
     t.coarse = (unsigned char)coarse_flag;
+    t.tail = tail ? 1 : 0;
     out->push_back(t);
   };
   if (coarse) {
@@ -161,38 +173,42 @@ void enqueue_cycle(BatchPlan& B, Sched& Sc) {
   BMember* mem = B.d_mem.as<BMember>();
   double* part = Sc.partials.as<double>();
   int* active = B.d_active.as<int>();
-  cudaStream_t s = B.stream;
-  const int T = kBThreads;
   auto S = [&](int l) { return tiles + Sc.off[l]; };
-  auto N = [&](int l) { return (unsigned)Sc.cnt[l]; };
   long long launches = 0;
-  kb_xupdate<<<N(0), T, 0, s>>>(S(0), lv, mem);
-  kb_outer<<<N(0), T, 0, s>>>(S(0), lv, mem, part, active);
-  kb_apply_pq<<<N(0), T, 0, s>>>(S(0), lv, mem, part);
-  kb_update<<<N(0), T, 0, s>>>(S(0), lv, mem, part);
-  launches += 4;
+  // programmatic serialization, as in launch_dep: every kernel of the cycle
+  // waits for its predecessor before its first read of changing memory
+  auto go = [&](int l, auto kern, auto... args) {
+    launch_dep(&B.cx, dim3((unsigned)Sc.cnt[l]), dim3(kBThreads), 0, kern, S(l), lv, args...);
+    ++launches;
+  };
+  const BMember* cmem = mem;
+  go(0, kb_xupdate, cmem);
+  go(0, kb_outer, mem, part, active);
+  go(0, kb_apply_pq, mem, part);
+  go(0, kb_update, mem, part);
   for (int l = 0; l + 1 < Sc.lmax; ++l) {
     for (int q = 0; q < B.prm.pre; ++q) {
-      kb_smooth<KT><<<N(l), T, 0, s>>>(S(l), lv, mem, 0, q == 0 ? 1 : 0);
-      kb_smooth<KT><<<N(l), T, 0, s>>>(S(l), lv, mem, 1, 0);
-      launches += 2;
+      go(l, kb_smooth<KT>, cmem, 0, q == 0 ? 1 : 0);
+      go(l, kb_smooth<KT>, cmem, 1, 0);
     }
-    kb_residual<KT><<<N(l), T, 0, s>>>(S(l), lv, mem);
-    kb_restrict<KT><<<N(l + 1), T, 0, s>>>(S(l + 1), lv, mem, B.prm.coarse_sweeps);
-    launches += 2;
+    go(l, kb_residual<KT>, cmem);
+    go(l + 1, kb_restrict<KT>, cmem, B.prm.coarse_sweeps);
+  }
+  if (Sc.ntails > 0) {
+    PDEB_CUDA(cudaFuncSetAttribute(kb_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCvSmem));
+    launch_dep(&B.cx, dim3((unsigned)Sc.ntails), dim3(kBTailThreads + 32), B.tail_smem, kb_tail,
+               (const BTail*)B.d_tails.as<BTail>(), (const int*)Sc.tails.as<int>(), mem, B.prm.pre, B.prm.post);
+    ++launches;
   }
   for (int l = Sc.lmax - 2; l >= 0; --l) {
-    kb_prolong<<<N(l), T, 0, s>>>(S(l), lv, mem);
-    ++launches;
+    go(l, kb_prolong, cmem);
     for (int q = 0; q < B.prm.post; ++q) {
-      kb_smooth<KT><<<N(l), T, 0, s>>>(S(l), lv, mem, 1, 0);
-      kb_smooth<KT><<<N(l), T, 0, s>>>(S(l), lv, mem, 0, 0);
-      launches += 2;
+      go(l, kb_smooth<KT>, cmem, 1, 0);
+      go(l, kb_smooth<KT>, cmem, 0, 0);
     }
   }
-  kb_rz<<<N(0), T, 0, s>>>(S(0), lv, mem, part);
-  kb_pupdate<<<N(0), T, 0, s>>>(S(0), lv, mem);
-  launches += 2;
+  go(0, kb_rz, mem, part);
+  go(0, kb_pupdate, cmem);
   Sc.launches = launches;
   PDEB_CUDA(cudaGetLastError());
 }
@@ -215,16 +231,23 @@ std::unique_ptr<Sched> make_sched(BatchPlan& B, const std::vector<int>* subset) 
     subset = &all_m;
   }
   Sc->members = (int)subset->size();
-  for (int m : *subset) Sc->lmax = std::max(Sc->lmax, B.nlev[m]);
+  // levels of a member that have tiles: up to its tail's first level
+  auto levels_of = [&](int m) { return B.tail_lev[m] >= 0 ? B.tail_lev[m] + 1 : B.nlev[m]; };
+  std::vector<int> tails;
+  for (int m : *subset) {
+    Sc->lmax = std::max(Sc->lmax, levels_of(m));
+    if (B.tail_lev[m] >= 0) tails.push_back(B.tail_rec[m]);
+  }
   Sc->tile0.assign(B.count, 0);
   Sc->ntiles.assign(B.count, 0);
   std::vector<std::vector<BTile>> per(Sc->lmax);
   for (int m : *subset) {
-    for (int l = 0; l < B.nlev[m]; ++l) {
+    for (int l = 0; l < levels_of(m); ++l) {
       const int rec = B.lev0[m] + l;
       const BLevel& L = B.levels[rec];
+      const bool tail = l == B.tail_lev[m];
       if (l == 0) Sc->tile0[m] = (int)per[0].size();
-      make_tiles(L.g, L.coarsest != 0, B.prm, rec, m, &per[l]);
+      make_tiles(L.g, L.coarsest != 0 && !tail, tail, B.prm, rec, m, &per[l]);
       if (l == 0) Sc->ntiles[m] = (int)per[0].size() - Sc->tile0[m];
     }
   }
@@ -240,6 +263,12 @@ std::unique_ptr<Sched> make_sched(BatchPlan& B, const std::vector<int>* subset) 
   Sc->tiles = Buf(sizeof(BTile) * all.size(), B.stream);
   PDEB_CUDA(cudaMemcpyAsync(Sc->tiles.as<void>(), all.data(), sizeof(BTile) * all.size(), cudaMemcpyHostToDevice,
                             B.stream));
+  Sc->ntails = (int)tails.size();
+  if (Sc->ntails) {
+    Sc->tails = Buf(sizeof(int) * tails.size(), B.stream);
+    PDEB_CUDA(cudaMemcpyAsync(Sc->tails.as<void>(), tails.data(), sizeof(int) * tails.size(), cudaMemcpyHostToDevice,
+                              B.stream));
+  }
   Sc->partials = Buf(sizeof(double) * (size_t)Sc->cnt[0], B.stream);
   PDEB_CUDA(cudaStreamSynchronize(B.stream));
   if (B.use_graph) {
@@ -408,6 +437,159 @@ void fill_hierarchy_k(BatchPlan& B, KT* kh0, float* k32, const double* k64) {
   PDEB_CUDA(cudaStreamSynchronize(B.stream));  // recs is released on return
 }
 
+// Transfer tables of the members whose coarse closure factors are per face, and
+// their places in the level records.
+void build_taps(BatchPlan& B) {
+  std::map<std::tuple<int, int, double, double>, int> seen;
+  std::vector<TapKey> keys;
+  size_t nr = 0, np = 0;
+  auto key_of = [&](int n, int nc, double lo, double hi) {
+    const auto k = std::make_tuple(n, nc, lo, hi);
+    const auto at = seen.find(k);
+    if (at != seen.end()) return at->second;
+    const int id = (int)keys.size();
+    keys.push_back(TapKey{n, nc, lo, hi, nr, np});
+    nr += nc;
+    np += n;
+    seen.emplace(k, id);
+    return id;
+  };
+  std::vector<int> axis_key(3 * B.levels.size(), -1);  // of the pair (prev, level)
+  for (auto& L : B.levels) L.pt_f32 = 0;
+  for (int m = 0; m < B.count; ++m) {
+    ExtCoef e;
+    bool scalar = true;
+    for (int l = 1; l < B.nlev[m]; ++l) scalar = scalar && ext_coef(B.levels[B.lev0[m] + l].g, &e);
+    if (!scalar) continue;
+    for (int l = 1; l < B.nlev[m]; ++l) {
+      const int r = B.lev0[m] + l;
+      const GridDev &f = B.levels[r - 1].g, &g = B.levels[r].g;
+      ext_coef(g, &e);
+      const int nf[3] = {f.nx, f.ny, f.nz}, nc[3] = {g.nx, g.ny, g.nz};
+      auto whole = [](double w) { return w == 0.0 || w == 1.0; };
+      bool f32 = true;
+      for (int a = 0; a < f.dim; ++a) {
+        axis_key[3 * r + a] = key_of(nf[a], nc[a], e.lo[a], e.hi[a]);
+        f32 = f32 && (nc[a] == nf[a] || 2 * nc[a] - 1 == nf[a]) && whole(e.lo[a]) && whole(e.hi[a]);
+      }
+      B.levels[r - 1].pt_f32 = f32;
+    }
+  }
+  for (auto& L : B.levels)
+    for (int a = 0; a < 3; ++a) {
+      L.rt[a] = nullptr;
+      L.pt[a] = nullptr;
+    }
+  if (keys.empty()) return;
+  B.d_taps = Buf(sizeof(RestrictTap) * nr + sizeof(ProlongTap) * np, B.stream);
+  RestrictTap* rt = B.d_taps.as<RestrictTap>();
+  ProlongTap* pt = reinterpret_cast<ProlongTap*>(rt + nr);
+  for (size_t r = 0; r < B.levels.size(); ++r)
+    for (int a = 0; a < 3; ++a) {
+      const int k = axis_key[3 * r + a];
+      if (k < 0) continue;
+      B.levels[r].rt[a] = rt + keys[k].r;
+      B.levels[r - 1].pt[a] = pt + keys[k].p;
+    }
+  Buf dk(sizeof(TapKey) * keys.size(), B.stream);
+  PDEB_CUDA(cudaMemcpyAsync(dk.as<void>(), keys.data(), sizeof(TapKey) * keys.size(), cudaMemcpyHostToDevice, B.stream));
+  kb_taps<<<(unsigned)keys.size(), 128, 0, B.stream>>>(dk.as<TapKey>(), rt, pt);
+  PDEB_CUDA(cudaGetLastError());
+  PDEB_CUDA(cudaStreamSynchronize(B.stream));  // keys is released on return
+}
+
+// Tails of the members whose coarse closure factors are per face and whose
+// coarsest level is small (the others run level by level to the coarsest
+// solve of kb_restrict).
+void build_tails(BatchPlan& B) {
+  B.tail_lev.assign(B.count, -1);
+  B.tail_rec.assign(B.count, -1);
+  std::vector<BTail> tails;
+  std::vector<CvGeo> geo;
+  std::vector<int> geo0;
+  std::vector<size_t> image_at, map_at;
+  size_t images = 0, maps = 0;
+  int max_lev = 0, max_coarse = 0;
+  for (int m = 0; m < B.count; ++m) {
+    const BLevel* L = &B.levels[B.lev0[m]];
+    const int n = B.nlev[m];
+    auto interior = [](const GridDev& g) { return (long long)(g.nx - 2) * (g.ny - 2) * (g.dim == 3 ? g.nz - 2 : 1); };
+    if (interior(L[n - 1].g) > kCvMaxCoarse) continue;
+    int first = std::max(0, n - kCvMaxLevels);
+    while (first < n && L[first].g.n > kBTailNodes) ++first;
+    if (first == n || (n > 1 && !L[1].rt[0])) continue;
+    std::vector<GridDev> gs;
+    for (int l = first; l < n; ++l) gs.push_back(L[l].g);
+    std::vector<CvGeo> q(n - first);
+    const CvLayout lay = cv_layout<float>(gs.data(), n - first, 1, 0, q.data());
+    if (lay.total > kCvSmem) continue;
+    for (int l = first; l < n; ++l) {
+      CvGeo& c = q[l - first];
+      ExtCoef e;
+      ext_coef(L[l].g, &e);
+      for (int a = 0; a < 3; ++a) {
+        c.lo[a] = e.lo[a];
+        c.hi[a] = e.hi[a];
+        c.rt[a] = L[l].rt[a];
+        c.pt[a] = L[l].pt[a];
+      }
+    }
+    BTail t{};
+    t.rhs = L[first].b;
+    t.x = L[first].x;
+    t.image_bytes = (unsigned)lay.image;
+    t.smem_bytes = (unsigned)lay.total;
+    t.nlev = n - first;
+    t.ncoarse = (int)interior(L[n - 1].g);
+    t.member = m;
+    t.level = B.lev0[m] + first;
+    image_at.push_back(images);
+    map_at.push_back(maps);
+    images += (lay.image + 127) / 128 * 128;
+    maps += (size_t)t.ncoarse * t.ncoarse;
+    geo0.push_back((int)geo.size());
+    geo.insert(geo.end(), q.begin(), q.end());
+    B.tail_lev[m] = first;
+    B.tail_rec[m] = (int)tails.size();
+    tails.push_back(t);
+    B.tail_smem = std::max(B.tail_smem, t.smem_bytes);
+    max_lev = std::max(max_lev, t.nlev);
+    max_coarse = std::max(max_coarse, t.ncoarse);
+  }
+  if (tails.empty()) return;
+  B.d_tail_images = Buf(images + sizeof(double) * maps, B.stream);
+  unsigned char* im = B.d_tail_images.as<unsigned char>();
+  for (size_t q = 0; q < tails.size(); ++q) {
+    tails[q].image = im + image_at[q];
+    tails[q].map = reinterpret_cast<double*>(im + images) + map_at[q];
+  }
+  B.d_tails = Buf(sizeof(BTail) * tails.size(), B.stream);
+  PDEB_CUDA(cudaMemcpyAsync(B.d_tails.as<void>(), tails.data(), sizeof(BTail) * tails.size(), cudaMemcpyHostToDevice,
+                            B.stream));
+  Buf dgeo(sizeof(CvGeo) * geo.size() + sizeof(int) * geo0.size(), B.stream);
+  int* dgeo0 = reinterpret_cast<int*>(dgeo.as<CvGeo>() + geo.size());
+  PDEB_CUDA(cudaMemcpyAsync(dgeo.as<void>(), geo.data(), sizeof(CvGeo) * geo.size(), cudaMemcpyHostToDevice, B.stream));
+  PDEB_CUDA(cudaMemcpyAsync(dgeo0, geo0.data(), sizeof(int) * geo0.size(), cudaMemcpyHostToDevice, B.stream));
+  const BLevel* lv = B.d_levels.as<BLevel>();
+  auto fill = [&](auto kt) {
+    using KT = decltype(kt);
+    // at most 65535 tails per launch row
+    for (size_t q = 0; q < tails.size(); q += 65535) {
+      const unsigned cnt = (unsigned)std::min<size_t>(65535, tails.size() - q);
+      kb_tail_image<KT><<<dim3(max_lev, cnt), 256, 0, B.stream>>>(B.d_tails.as<BTail>() + q, dgeo.as<CvGeo>(), dgeo0 + q,
+                                                                  lv);
+      kb_tail_map<KT><<<dim3(max_coarse, cnt), kCvMaxCoarse, 0, B.stream>>>(B.d_tails.as<BTail>() + q, lv,
+                                                                           B.prm.coarse_sweeps);
+    }
+  };
+  if (B.bf16)
+    fill(__nv_bfloat16{});
+  else
+    fill(float{});
+  PDEB_CUDA(cudaGetLastError());
+  PDEB_CUDA(cudaStreamSynchronize(B.stream));  // the host tables and dgeo are released on return
+}
+
 void create_plan(BatchPlan& B, const pdeb200_problem* probs, int count, const pdeb200_batch_options* o) {
   if (!probs || count <= 0) throw StatusFailure{PDEB200_ERR_INVALID, "empty batch"};
   B.count = count;
@@ -425,6 +607,7 @@ void create_plan(BatchPlan& B, const pdeb200_problem* probs, int count, const pd
   B.cx.dev = o->device;
   B.cx.stream = B.stream;
   B.cx.own_stream = nullptr;
+  B.cx.pdl = std::getenv("PDEB200_NO_PDL") == nullptr;
   PDEB_CUDA(cudaEventCreate(&B.ev0));
   PDEB_CUDA(cudaEventCreate(&B.ev1));
   PDEB_CUDA(cudaMallocHost(&B.h_active, sizeof(int)));
@@ -577,6 +760,7 @@ void create_plan(BatchPlan& B, const pdeb200_problem* probs, int count, const pd
     M.q = a32 + q_off[m];
     M.e = a32 + e_off[m];
   }
+  build_taps(B);
   B.d_levels = Buf(sizeof(BLevel) * B.levels.size(), B.stream);
   PDEB_CUDA(cudaMemcpyAsync(B.d_levels.as<void>(), B.levels.data(), sizeof(BLevel) * B.levels.size(),
                             cudaMemcpyHostToDevice, B.stream));
@@ -584,6 +768,7 @@ void create_plan(BatchPlan& B, const pdeb200_problem* probs, int count, const pd
     fill_hierarchy_k<__nv_bfloat16>(B, reinterpret_cast<__nv_bfloat16*>(akh), k32, k64);
   else
     fill_hierarchy_k<float>(B, reinterpret_cast<float*>(akh), k32, k64);
+  build_tails(B);
   B.d_mem = Buf(sizeof(BMember) * count, B.stream);
   B.d_active = Buf(sizeof(int), B.stream);
   PDEB_CUDA(cudaStreamSynchronize(B.stream));
@@ -870,6 +1055,7 @@ pdeb200_status pdeb200_batch_solve(pdeb200_batch* b, double tol, pdeb200_report*
     stats->tiles_level0 = B.full ? B.full->cnt[0] : 0;
     stats->nodes = B.nodes;
     size_t bytes = B.a64.bytes() + B.a32.bytes() + B.akh.bytes() + B.d_levels.bytes() + B.d_mem.bytes() +
+                   B.d_tails.bytes() + B.d_taps.bytes() + B.d_tail_images.bytes() +
                    (B.full ? B.full->tiles.bytes() + B.full->partials.bytes() : 0);
     for (const auto& P : B.probs)
       for (const auto& buf : P.owned) bytes += buf.bytes();

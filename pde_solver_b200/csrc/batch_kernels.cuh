@@ -23,6 +23,7 @@
 
 #include <type_traits>
 
+#include "cluster_vcycle.cuh"
 #include "kernels.cuh"
 
 namespace pdeb {
@@ -44,6 +45,9 @@ struct BLevel {
   float* x;                                       // correction (level 0: z = M r)
   float* b;                                       // right-hand side (level 0: PCG residual r)
   float* r;                                       // residual scratch
+  const RestrictTap* rt[3];                       // onto this level from the finer one (null: closures per node)
+  const ProlongTap* pt[3];                        // to this level from the coarser one
+  int pt_f32;                                     // weights of pt are 0, 1/2 and 1
 };
 
 // Per-member solver state and level-0 vectors.
@@ -85,8 +89,21 @@ struct alignas(16) BTile {
   unsigned short w, h;   // extent in nodes
   unsigned char lw;      // log2 of the padded row width (w <= 1 << lw)
   unsigned char coarse;  // whole-grid tile of a coarsest level
-  unsigned char pad[2];
+  unsigned char tail;    // on the level that kb_tail takes over: no smoothing, residual or prolongation
+  unsigned char pad;
 };
+
+// The lower levels of a member's V-cycle, run by one block (kb_tail).
+struct BTail {
+  const unsigned char* image;
+  const float* rhs;
+  float* x;
+  const double* map;
+  unsigned image_bytes, smem_bytes;
+  int nlev, ncoarse, member, level;  // level: record of the first of them
+};
+constexpr int kBTailNodes = 1200;     // largest level of a tail
+constexpr int kBTailThreads = 256;    // that update nodes; one more warp controls
 
 // Visits the (i,j) columns of tile T that this thread owns: thread t takes
 // column t & (W-1) of row t >> lw (W = 1 << lw), so a warp covers 32
@@ -354,6 +371,8 @@ __global__ void __launch_bounds__(kBThreads) kb_rhs(const BTile* __restrict__ ti
 // x64 += e for members about to take an outer step with a pending correction.
 __global__ void __launch_bounds__(kBThreads) kb_xupdate(const BTile* __restrict__ tiles, const BLevel* __restrict__ lv,
                                                         const BMember* mem) {
+  grid_dep_wait();
+  grid_dep_release();
   const BTile T = tiles[blockIdx.x];
   const BMember* m = mem + T.member;
   if (bstate(m) != kBNeedOuter || !__ldcg(&m->e_valid)) return;
@@ -371,6 +390,8 @@ __global__ void __launch_bounds__(kBThreads) kb_xupdate(const BTile* __restrict_
 // Outer FP64 residual r = b - A x; the FP32 copy is the inner right-hand side.
 __global__ void __launch_bounds__(kBThreads) kb_outer(const BTile* __restrict__ tiles, const BLevel* __restrict__ lv,
                                                       BMember* mem, double* partials, int* active) {
+  grid_dep_wait();
+  grid_dep_release();
   const BTile T = tiles[blockIdx.x];
   BMember* m = mem + T.member;
   if (bstate(m) != kBNeedOuter) return;
@@ -405,6 +426,8 @@ __global__ void __launch_bounds__(kBThreads) kb_outer(const BTile* __restrict__ 
 __global__ void __launch_bounds__(kBThreads, 5) kb_apply_pq(const BTile* __restrict__ tiles,
                                                          const BLevel* __restrict__ lv, BMember* mem,
                                                          double* partials) {
+  grid_dep_wait();
+  grid_dep_release();
   const BTile T = tiles[blockIdx.x];
   BMember* m = mem + T.member;
   if (bstate(m) != kBInnerRun) return;
@@ -443,6 +466,8 @@ __global__ void __launch_bounds__(kBThreads, 5) kb_apply_pq(const BTile* __restr
 // e (+)= alpha p, r -= alpha q, sum r.r in FP64.
 __global__ void __launch_bounds__(kBThreads) kb_update(const BTile* __restrict__ tiles, const BLevel* __restrict__ lv,
                                                        BMember* mem, double* partials) {
+  grid_dep_wait();
+  grid_dep_release();
   const BTile T = tiles[blockIdx.x];
   BMember* m = mem + T.member;
   if (bstate(m) != kBInnerRun) return;
@@ -469,6 +494,8 @@ __global__ void __launch_bounds__(kBThreads) kb_update(const BTile* __restrict__
 // sum r.z in FP64 (starts a new inner solve or gives beta).
 __global__ void __launch_bounds__(kBThreads) kb_rz(const BTile* __restrict__ tiles, const BLevel* __restrict__ lv,
                                                    BMember* mem, double* partials) {
+  grid_dep_wait();
+  grid_dep_release();
   const BTile T = tiles[blockIdx.x];
   BMember* m = mem + T.member;
   if (!vcycle_state(bstate(m))) return;
@@ -488,6 +515,8 @@ __global__ void __launch_bounds__(kBThreads) kb_rz(const BTile* __restrict__ til
 // p = z + beta p (p = z when the inner solve starts).
 __global__ void __launch_bounds__(kBThreads) kb_pupdate(const BTile* __restrict__ tiles,
                                                         const BLevel* __restrict__ lv, const BMember* mem) {
+  grid_dep_wait();
+  grid_dep_release();
   const BTile T = tiles[blockIdx.x];
   const BMember* m = mem + T.member;
   if (bstate(m) != kBInnerRun) return;
@@ -510,8 +539,10 @@ __global__ void __launch_bounds__(kBThreads) kb_pupdate(const BTile* __restrict_
 template <typename KT>
 __global__ void __launch_bounds__(kBThreads, 8) kb_smooth(const BTile* __restrict__ tiles, const BLevel* __restrict__ lv,
                                                        const BMember* mem, int color, int from_zero) {
+  grid_dep_wait();
+  grid_dep_release();
   const BTile T = tiles[blockIdx.x];
-  if (T.coarse) return;
+  if (T.coarse || T.tail) return;
   if (!vcycle_state(bstate(mem + T.member))) return;
   const BLevel& L = lv[T.lev];
   float* __restrict__ x = L.x;
@@ -570,8 +601,10 @@ __global__ void __launch_bounds__(kBThreads, 8) kb_smooth(const BTile* __restric
 template <typename KT>
 __global__ void __launch_bounds__(kBThreads, kBMinBlocks) kb_residual(const BTile* __restrict__ tiles,
                                                          const BLevel* __restrict__ lv, const BMember* mem) {
+  grid_dep_wait();
+  grid_dep_release();
   const BTile T = tiles[blockIdx.x];
-  if (T.coarse) return;
+  if (T.coarse || T.tail) return;
   if (!vcycle_state(bstate(mem + T.member))) return;
   const BLevel& L = lv[T.lev];
   const float* __restrict__ x = L.x;
@@ -724,6 +757,8 @@ template <typename KT>
 __global__ void __launch_bounds__(kBThreads, 4) kb_restrict(const BTile* __restrict__ tiles,
                                                          const BLevel* __restrict__ lv, const BMember* mem,
                                                          int coarse_sweeps) {
+  grid_dep_wait();
+  grid_dep_release();
   const BTile T = tiles[blockIdx.x];
   if (!vcycle_state(bstate(mem + T.member))) return;
   const BLevel& C = lv[T.lev];
@@ -740,6 +775,88 @@ __global__ void __launch_bounds__(kBThreads, 4) kb_restrict(const BTile* __restr
   const bool fast = xm <= 1 && ym <= 1 && zmarch;
   const int fnx = F.g.nx;
   const long long fsxy = F.g.sxy;
+  if (C.rt[0]) {
+    // Taps per axis (boundary closures included): a column's taps are loaded
+    // once and the sums of fine planes are shared by the coarse planes they
+    // feed. FP32 where the weights are 1/4, 1/2, 1/4, FP64 elsewhere (closures
+    // that fold in, pairs not nested). The form with a walk over the boundary
+    // neighbours per node, below, took 64 us per launch of the batch named at
+    // kb_tail, this one 24.
+    auto plain = [](const RestrictTap& t) { return t.w[0] == 0.25 && t.w[1] == 0.5 && t.w[2] == 0.25; };
+    const bool nested = xm == 1 && ym == 1 && (gc.dim != 3 || 2 * gc.nz - 1 == F.g.nz);
+    tile_columns(T, [&](int I, int J) {
+      const RestrictTap& ax = C.rt[0][I];
+      const RestrictTap& ay = C.rt[1][J];
+      const float* base = rf + (long long)ay.i0 * fnx + ax.i0;
+      auto plane64 = [&](int kf) -> double {
+        const float* p = base + (long long)kf * fsxy;
+        double v = 0.0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          if (ay.w[b] == 0.0) continue;
+          const float* q = p + b * fnx;
+          double s = ax.w[0] * double(q[0]);
+#pragma unroll
+          for (int a = 1; a < 4; ++a)
+            if (ax.w[a] != 0.0) s += ax.w[a] * double(q[a]);
+          v += ay.w[b] * s;
+        }
+        return v;
+      };
+      if (nested && plain(ax) && plain(ay)) {
+        auto plane = [&](int kf) -> float {
+          const float* p = base + (long long)kf * fsxy;
+          auto row = [](const float* q) { return 0.25f * q[0] + 0.5f * q[1] + 0.25f * q[2]; };
+          return 0.25f * row(p) + 0.5f * row(p + fnx) + 0.25f * row(p + 2 * fnx);
+        };
+        if (gc.dim != 3) {
+          bc[bid(gc, I, J, 0)] = plane(0);
+          return;
+        }
+        float below = plane(2 * T.z0 - 1);
+        for (int K = T.z0; K < T.z1; ++K) {
+          const float mid = plane(2 * K), above = plane(2 * K + 1);
+          float v = 0.25f * below + 0.5f * mid + 0.25f * above;
+          if (K == 1 || K == gc.nz - 2) {
+            const RestrictTap& az = C.rt[2][K];
+            if (!plain(az))
+              v = float(az.w[0] * plane64(2 * K - 1) + az.w[1] * plane64(2 * K) + az.w[2] * plane64(2 * K + 1));
+          }
+          bc[bid(gc, I, J, K)] = v;
+          below = above;
+        }
+        return;
+      }
+      if (gc.dim != 3) {
+        bc[bid(gc, I, J, 0)] = float(plane64(0));
+        return;
+      }
+      double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;  // sums of planes at .. at + 3, the first `have` of them
+      int at = 0, have = 0;
+      for (int K = T.z0; K < T.z1; ++K) {
+        const RestrictTap& az = C.rt[2][K];
+        while (have > 0 && at < az.i0) {
+          s0 = s1;
+          s1 = s2;
+          s2 = s3;
+          ++at;
+          --have;
+        }
+        if (have == 0) at = az.i0;
+        if (have <= 0 && az.w[0] != 0.0) s0 = plane64(at);
+        if (have <= 1 && az.w[1] != 0.0) s1 = plane64(at + 1);
+        if (have <= 2 && az.w[2] != 0.0) s2 = plane64(at + 2);
+        if (have <= 3 && az.w[3] != 0.0) s3 = plane64(at + 3);
+        have = az.w[0] == 0.0 ? 0 : (az.w[1] == 0.0 ? 1 : (az.w[2] == 0.0 ? 2 : (az.w[3] == 0.0 ? 3 : 4)));
+        bc[bid(gc, I, J, K)] = float(az.w[0] * s0 + az.w[1] * s1 + az.w[2] * s2 + az.w[3] * s3);
+      }
+    });
+    if (T.coarse) {
+      __syncthreads();
+      bcoarse_solve<KT>(C, coarse_sweeps);
+    }
+    return;
+  }
   tile_columns(T, [&](int I, int J) {
     if (fast) {
       const int fi = (xm == 1 ? 2 * I : I) - 1, fj = (ym == 1 ? 2 * J : J) - 1;
@@ -788,8 +905,10 @@ __global__ void __launch_bounds__(kBThreads, 4) kb_restrict(const BTile* __restr
 // x_l += P Ext(x_{l+1}) on level-l tiles of members with a coarser level.
 __global__ void __launch_bounds__(kBThreads, 5) kb_prolong(const BTile* __restrict__ tiles, const BLevel* __restrict__ lv,
                                                         const BMember* mem) {
+  grid_dep_wait();
+  grid_dep_release();
   const BTile T = tiles[blockIdx.x];
-  if (T.coarse) return;
+  if (T.coarse || T.tail) return;
   if (!vcycle_state(bstate(mem + T.member))) return;
   const BLevel& F = lv[T.lev];
   const BLevel& C = lv[F.next];
@@ -799,6 +918,56 @@ __global__ void __launch_bounds__(kBThreads, 5) kb_prolong(const BTile* __restri
   float* __restrict__ xf = F.x;
   const int xmode = map_mode(gf.nx, gc.nx), ymode = map_mode(gf.ny, gc.ny);
   const int zmode = gf.dim == 3 ? map_mode(gf.nz, gc.nz) : 0;
+  if (F.pt[0]) {
+    // Taps per axis (boundary extension included), the x-y sum of the two
+    // coarse planes around a fine one kept while marching. FP32 where every
+    // weight is 0, 1/2 or 1, else FP64. With the extension chains and positions
+    // evaluated per node, below, took 26 us per launch of the batch named
+    // at kb_tail, this one 14.
+    auto columns = [&](auto zero) {
+      using A = decltype(zero);
+      tile_columns(T, [&](int i, int j) {
+        const ProlongTap& tx = F.pt[0][i];
+        const ProlongTap& ty = F.pt[1][j];
+        const A w00 = A(ty.w[0] * tx.w[0]), w10 = A(ty.w[0] * tx.w[1]);
+        const A w01 = A(ty.w[1] * tx.w[0]), w11 = A(ty.w[1] * tx.w[1]);
+        const int o00 = ty.i[0] * gc.nx + tx.i[0], o10 = ty.i[0] * gc.nx + tx.i[1];
+        const int o01 = ty.i[1] * gc.nx + tx.i[0], o11 = ty.i[1] * gc.nx + tx.i[1];
+        auto plane = [&](int K) -> A {
+          const float* p = xc + (long long)K * gc.sxy;
+          return (w00 * A(p[o00]) + w10 * A(p[o10])) + (w01 * A(p[o01]) + w11 * A(p[o11]));
+        };
+        if (gf.dim != 3) {
+          const long long id = bid(gf, i, j, 0);
+          xf[id] = float(A(xf[id]) + plane(0));
+          return;
+        }
+        int ka = -1, kb = -1;
+        A va = A(0), vb = A(0);
+        auto at = [&](int K) -> A {
+          if (K == kb) return vb;
+          if (K == ka) return va;
+          ka = kb;
+          va = vb;
+          kb = K;
+          vb = plane(K);
+          return vb;
+        };
+        for (int k = T.z0; k < T.z1; ++k) {
+          const ProlongTap& tz = F.pt[2][k];
+          A v = A(tz.w[0]) * at(tz.i[0]);
+          if (tz.w[1] != 0.0) v += A(tz.w[1]) * at(tz.i[1]);
+          const long long id = bid(gf, i, j, k);
+          xf[id] = float(A(xf[id]) + v);
+        }
+      });
+    };
+    if (F.pt_f32)
+      columns(float(0));
+    else
+      columns(double(0));
+    return;
+  }
   if (xmode <= 1 && ymode <= 1 && zmode <= 1) {
     // nested 2:1 or identity in every dimension: interpolation weights are 1
     // or 1/2, in FP32, loading only the coarse values a node uses
@@ -894,6 +1063,64 @@ __global__ void __launch_bounds__(kBThreads, 5) kb_prolong(const BTile* __restri
       const long long id = bid(gf, i, j, k);
       xf[id] = float(double(xf[id]) + v);
     }
+  });
+}
+
+// The lower levels of the members' V-cycles, one block per member, in its
+// shared memory (cv_cycle): a level of at most kBTailNodes nodes and all below
+// it are one launch for all members instead of twelve per level, and the
+// coarsest solve is one small matrix. Fixed for a member whatever its batch, so
+// its numbers do not depend on the other members.
+// 56 2D and 8 3D members (sides 33..257 and 17..65): 22.8 us per cycle instead
+// of about four levels of twelve launches each (6 to 9 us a launch) and the
+// coarsest solves; with it and the launches overlapped (grid_dep_wait) the
+// batch takes 20.4 ms instead of 26.5, with the transfer taps 16.5.
+__global__ void __launch_bounds__(kBTailThreads + 32) kb_tail(const BTail* __restrict__ tails,
+                                                              const int* __restrict__ list, BMember* mem, int pre,
+                                                              int post) {
+  const BTail t = tails[list[blockIdx.x]];
+  BMember* m = mem + t.member;
+  if (cv_cycle<float, kBTailThreads>(t.image, t.image_bytes, t.smem_bytes, t.nlev, t.rhs, t.x, pre, post, t.map,
+                                     t.ncoarse, [&]() { return vcycle_state(bstate(m)); }))
+    m->state = kBNeedOuter;  // a wait ran out: restart from the current refinement
+}
+
+// Transfer taps of one axis of a level pair, shared by the pairs of equal sizes
+// and closure factors: block q fills the tables of key q.
+struct TapKey {
+  int n, nc;
+  double lo, hi;
+  size_t r, p;  // first entries
+};
+__global__ void kb_taps(const TapKey* __restrict__ keys, RestrictTap* __restrict__ rt, ProlongTap* __restrict__ pt) {
+  const TapKey k = keys[blockIdx.x];
+  for (int I = threadIdx.x; I < k.nc; I += blockDim.x) rt[k.r + I] = restrict_tap(I, k.n, k.nc, k.lo, k.hi);
+  for (int i = threadIdx.x; i < k.n; i += blockDim.x) pt[k.p + i] = prolong_tap(i, k.n, k.nc, k.lo, k.hi);
+}
+
+// Images of the tails' levels (level blockIdx.x of tail blockIdx.y) and columns
+// of their coarsest maps.
+template <typename KT>
+__global__ void __launch_bounds__(256) kb_tail_image(const BTail* __restrict__ tails, const CvGeo* __restrict__ geo,
+                                                     const int* __restrict__ geo0, const BLevel* __restrict__ lv) {
+  const BTail t = tails[blockIdx.y];
+  const int l = blockIdx.x;
+  if (l >= t.nlev) return;
+  const BLevel& L = lv[t.level + l];
+  cv_write_image<float>(geo[geo0[blockIdx.y] + l], t.nlev, l, 0, const_cast<unsigned char*>(t.image),
+                        [&](int i, int j, int k) {
+                          return bstencil<float, KT>(L, static_cast<const KT*>(L.kh), i, j, k, bid(L.g, i, j, k), nullptr);
+                        });
+}
+
+template <typename KT>
+__global__ void __launch_bounds__(kCvMaxCoarse) kb_tail_map(const BTail* __restrict__ tails,
+                                                            const BLevel* __restrict__ lv, int sweeps) {
+  const BTail t = tails[blockIdx.y];
+  if ((int)blockIdx.x >= t.ncoarse) return;
+  const BLevel& L = lv[t.level + t.nlev - 1];
+  cv_map_column(L.g, sweeps, blockIdx.x, const_cast<double*>(t.map), [&](int i, int j, int k) {
+    return bstencil<double, KT>(L, static_cast<const KT*>(L.kh), i, j, k, bid(L.g, i, j, k), nullptr);
   });
 }
 

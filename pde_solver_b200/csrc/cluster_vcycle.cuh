@@ -138,13 +138,11 @@ __device__ __forceinline__ void cv_owner(const CvGeo& q, int layer, int& rank, i
   }
 }
 
-// The image of CTA blockIdx.x, level blockIdx.y: places and folded weights.
-template <class Coef, typename T>
-__global__ void __launch_bounds__(256) k_cv_image(const CvLevel<Coef, T>* __restrict__ lv, int nlev, size_t image,
-                                                  unsigned char* __restrict__ out) {
-  const int rank = blockIdx.x, l = blockIdx.y;
-  unsigned char* base = out + (size_t)rank * image;
-  const CvGeo q = lv[l].q;
+// Writes level l of CTA `rank`'s image at `base`: places and folded weights,
+// folded(i, j, k) being the folded stencil of an interior node.
+template <typename T, class Folded>
+__device__ __forceinline__ void cv_write_image(const CvGeo& q, int nlev, int l, int rank, unsigned char* base,
+                                               const Folded& folded) {
   CvSlab s;
   s.init(q, rank);
   const bool is3 = q.dim == 3;
@@ -174,7 +172,6 @@ __global__ void __launch_bounds__(256) k_cv_image(const CvLevel<Coef, T>* __rest
   }
   unsigned* tab = reinterpret_cast<unsigned*>(base + q.tab);
   T* w = reinterpret_cast<T*>(base + q.w);
-  const GridDev& g = lv[l].g;
   for (int t = threadIdx.x; t < 2 * cnt; t += blockDim.x) {
     const int p = t >= cnt, u = t - p * cnt, row = u / q.half, m = u - row * q.half;
     const int layer = row / q.H, jj = row - layer * q.H;
@@ -185,8 +182,7 @@ __global__ void __launch_bounds__(256) k_cv_image(const CvLevel<Coef, T>* __rest
       e = (unsigned)((layer + 1) * q.L + (is3 ? j * q.nx : 0) + i);
       if (layer == 0 && prev) e |= kClPrev;
       if (layer == s.n - 1 && next) e |= kClNext;
-      Stencil<T> st = lv[l].cf.template at<T>(g, ((long long)k * q.ny + j) * q.nx + i);
-      fold_faces<T>(g, i, j, k, st, nullptr);
+      const Stencil<T> st = folded(i, j, k);
       T* ws = w + (t >> 5) * (32 * kCvRows) + (t & 31);
       ws[0] = T(1) / st.c;
       ws[32] = st.xm;
@@ -200,6 +196,19 @@ __global__ void __launch_bounds__(256) k_cv_image(const CvLevel<Coef, T>* __rest
   }
 }
 
+// The image of CTA blockIdx.x, level blockIdx.y.
+template <class Coef, typename T>
+__global__ void __launch_bounds__(256) k_cv_image(const CvLevel<Coef, T>* __restrict__ lv, int nlev, size_t image,
+                                                  unsigned char* __restrict__ out) {
+  const int l = blockIdx.y;
+  const GridDev& g = lv[l].g;
+  cv_write_image<T>(lv[l].q, nlev, l, blockIdx.x, out + (size_t)blockIdx.x * image, [&](int i, int j, int k) {
+    Stencil<T> st = lv[l].cf.template at<T>(g, ((long long)k * g.ny + j) * g.nx + i);
+    fold_faces<T>(g, i, j, k, st, nullptr);
+    return st;
+  });
+}
+
 // One V-cycle of the image's nlev levels on rhs0, result in x0 (interior and
 // zero boundary).
 //
@@ -209,17 +218,19 @@ __global__ void __launch_bounds__(256) k_cv_image(const CvLevel<Coef, T>* __rest
 // 33^3 and below 47 us, where the launches and the single-block tail took
 // about 172 us; 129x97 and below 38 us (about 170); 51x39x30 and below 42 us (about
 // 290, restriction folds included).
-template <typename T>
-__global__ void __launch_bounds__(kCvThreads + 32) k_cluster_vcycle(const unsigned char* __restrict__ image,
-                                                                    unsigned image_bytes, unsigned smem_bytes, int nlev,
-                                                                    const T* __restrict__ rhs0, T* __restrict__ x0,
-                                                                    int pre, int post,
-                                                                    const double* __restrict__ coarse_map, int ncoarse,
-                                                                    Ctl* ctl) {
+//
+// NU threads update nodes, 32 more control. go(), called once the preceding
+// kernel has completed, tells whether to run. Returns true in one thread of a CTA
+// that lost a wait.
+template <typename T, int NU, class Go>
+__device__ __forceinline__ bool cv_cycle(const unsigned char* __restrict__ image, unsigned image_bytes,
+                                         unsigned smem_bytes, int nlev, const T* __restrict__ rhs0,
+                                         T* __restrict__ x0, int pre, int post, const double* __restrict__ coarse_map,
+                                         int ncoarse, const Go& go) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ unsigned long long mbs[2], mbi;
   const unsigned csize = cl_size(), rank = cl_rank();
-  constexpr int nu = kCvThreads;
+  constexpr int nu = NU;
   const int tid = threadIdx.x, lane = tid & 31;
   const bool control = tid >= nu;
   constexpr unsigned kT = sizeof(T);
@@ -293,7 +304,7 @@ __global__ void __launch_bounds__(kCvThreads + 32) k_cluster_vcycle(const unsign
   Here h = enter(0);
   grid_dep_wait();
   grid_dep_release();
-  if (ctl_skip(ctl)) return;  // the same in every CTA: the flag is not written while this kernel runs
+  if (!go()) return false;  // the same in every CTA
   {
     const T* src = rhs0 + (long long)(h.lo - 1) * h.L;
     for (int t = tid; t < 2 * h.cnt; t += blockDim.x) {
@@ -573,27 +584,37 @@ __global__ void __launch_bounds__(kCvThreads + 32) k_cluster_vcycle(const unsign
   __syncthreads();
   for (int t = tid; t < h.n * h.L; t += blockDim.x) x0[(long long)h.lo * h.L + t] = h.x[h.L + t];
   cl_leave(csize);
-  if (control && lane == 0 && dead) {
+  return control && lane == 0 && dead;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kCvThreads + 32) k_cluster_vcycle(const unsigned char* __restrict__ image,
+                                                                    unsigned image_bytes, unsigned smem_bytes, int nlev,
+                                                                    const T* __restrict__ rhs0, T* __restrict__ x0,
+                                                                    int pre, int post,
+                                                                    const double* __restrict__ coarse_map, int ncoarse,
+                                                                    Ctl* ctl) {
+  // the flag is not written while this kernel runs
+  if (cv_cycle<T, kCvThreads>(image, image_bytes, smem_bytes, nlev, rhs0, x0, pre, post, coarse_map, ncoarse,
+                              [&]() { return !ctl_skip(ctl); })) {
     ctl->status = PDEB200_ERR_TIMEOUT;
     ctl->done = 1;
   }
 }
 
-// Column `blockIdx.x` of the coarsest level's map: `sweeps` red-black sweeps
-// from zero for the unit right-hand side, in FP64 (map[col * n + row], interior
-// nodes in row-major order).
-template <class Coef>
-__global__ void __launch_bounds__(kCvMaxCoarse) k_coarse_map(GridDev g, Coef cf, int sweeps, double* __restrict__ map) {
+// Column `col` of the coarsest level's map: `sweeps` red-black sweeps from
+// zero for the unit right-hand side, in FP64 (map[col * n + row], interior nodes
+// in row-major order). folded(i, j, k) as in cv_write_image. One block of
+// kCvMaxCoarse threads.
+template <class Folded>
+__device__ __forceinline__ void cv_map_column(const GridDev& g, int sweeps, int col, double* __restrict__ map,
+                                              const Folded& folded) {
   __shared__ double sx[kCvMaxCoarse];
   const int ni = g.nx - 2, nj = g.ny - 2, nk = g.dim == 3 ? g.nz - 2 : 1, n = ni * nj * nk;
-  const int t = threadIdx.x, col = blockIdx.x;
+  const int t = threadIdx.x;
   const int i = t % ni, j = (t / ni) % nj, k = t / (ni * nj);
   Stencil<double> s{};
-  if (t < n) {
-    const int kk = g.dim == 3 ? k + 1 : 0;
-    s = cf.template at<double>(g, ((long long)kk * g.ny + j + 1) * g.nx + i + 1);
-    fold_faces<double>(g, i + 1, j + 1, kk, s, nullptr);
-  }
+  if (t < n) s = folded(i + 1, j + 1, g.dim == 3 ? k + 1 : 0);
   sx[t] = 0.0;
   __syncthreads();
   if (n == 1) sweeps = 1;  // the first sweep is the fixed point
@@ -613,6 +634,15 @@ __global__ void __launch_bounds__(kCvMaxCoarse) k_coarse_map(GridDev g, Coef cf,
     __syncthreads();
   }
   if (t < n) map[col * n + t] = sx[t];
+}
+
+template <class Coef>
+__global__ void __launch_bounds__(kCvMaxCoarse) k_coarse_map(GridDev g, Coef cf, int sweeps, double* __restrict__ map) {
+  cv_map_column(g, sweeps, blockIdx.x, map, [&](int i, int j, int k) {
+    Stencil<double> s = cf.template at<double>(g, ((long long)k * g.ny + j) * g.nx + i);
+    fold_faces<double>(g, i, j, k, s, nullptr);
+    return s;
+  });
 }
 
 // Restriction of one level pair as a launch: full weighting and the transpose
@@ -692,24 +722,23 @@ __global__ void __launch_bounds__(kBx* kBy) k_restrict_taps(LevelGeo gf, LevelGe
     if (have <= 1 && az.w[1] != 0.0) s1 = plane(at + 1);
     if (have <= 2 && az.w[2] != 0.0) s2 = plane(at + 2);
     if (have <= 3 && az.w[3] != 0.0) s3 = plane(at + 3);
-    have = az.w[3] != 0.0 ? 4 : (az.w[2] != 0.0 ? 3 : (az.w[1] != 0.0 ? 2 : 1));
+    have = az.w[0] == 0.0 ? 0 : (az.w[1] == 0.0 ? 1 : (az.w[2] == 0.0 ? 2 : (az.w[3] == 0.0 ? 3 : 4)));
     *out = T(az.w[0] * s0 + az.w[1] * s1 + az.w[2] * s2 + az.w[3] * s3);
   }
 }
 
-// ------------------------------------------------------------- host side
-
 // taps of coarse index I on one axis: full weighting plus the transpose of the
 // boundary extension (lo, hi: the closure factors of the axis's faces), interior fine nodes only
-inline RestrictTap restrict_tap(int I, int n, int nc, double lo, double hi) {
+__host__ __device__ inline RestrictTap restrict_tap(int I, int n, int nc, double lo, double hi) {
   RestrictTap t{{0, 0, 0, 0}, 0, 0};
   const int den = n - 1, m = nc - 1;
   auto full = [&](int J, int i) -> double {
     if (nc == n) return i == J ? 1.0 : 0.0;
-    const long long d = std::llabs((long long)i * m - (long long)J * den);
+    long long d = (long long)i * m - (long long)J * den;
+    d = d < 0 ? -d : d;
     return d < den ? double(m) / double(den) * (1.0 - double(d) / double(den)) : 0.0;
   };
-  // the first interior fine index with a weight of I, 0 or nc - 1 folded into I
+  // with the boundary indices 0 and nc - 1 folded into I
   auto weight = [&](int i) -> double {
     if (i < 1 || i > n - 2) return 0.0;
     double w = full(I, i);
@@ -717,15 +746,15 @@ inline RestrictTap restrict_tap(int I, int n, int nc, double lo, double hi) {
     if (I == nc - 2) w += hi * full(nc - 1, i);
     return w;
   };
-  int i0 = nc == n ? I : (int)std::floor(double(I - 1) * den / m);
+  int i0 = nc == n ? I : (int)floor(double(I - 1) * den / m);
   if (i0 < 1) i0 = 1;
-  while (i0 < n - 2 && weight(i0) == 0.0) ++i0;
+  while (i0 < n - 2 && full(I, i0) == 0.0) ++i0;
   t.i0 = i0;
   for (int q = 0; q < 4; ++q) t.w[q] = weight(i0 + q);
   return t;
 }
 
-inline ProlongTap prolong_tap(int i, int n, int nc, double lo, double hi) {
+__host__ __device__ inline ProlongTap prolong_tap(int i, int n, int nc, double lo, double hi) {
   ProlongTap t{{1.0, 0.0}, {0, 0}};
   int I0;
   double s;
@@ -745,6 +774,8 @@ inline ProlongTap prolong_tap(int i, int n, int nc, double lo, double hi) {
   }
   return t;
 }
+
+// ------------------------------------------------------------- host side
 
 // Places the levels q[0 .. n) (grids g) in shared memory; levels of at most
 // `single` interior nodes go to the first CTA alone.

@@ -200,3 +200,48 @@ def test_compaction_changes_no_numbers(batch_result, members):
         plain = b.read()
     for u, v in zip(compacted, plain):
         assert np.array_equal(u, v)
+
+
+# sides around the largest level that one block takes (1200 nodes), with and
+# without levels above it, nested and ragged, a single coarse node
+LOWER = [(5, 5, 1), (33, 33, 1), (40, 30, 1), (41, 30, 1), (50, 37, 1), (130, 77, 1), (5, 5, 5), (9, 9, 9), (12, 10, 10),
+         (11, 11, 10), (17, 17, 17), (29, 21, 18), (7, 40, 9)]
+
+
+@pytest.mark.parametrize("coef", ["divk", "const"])
+@pytest.mark.parametrize("bf16", [0, 1])
+def test_lower_levels_in_one_block_match_level_by_level(oracle_mod, coef, bf16):
+    # A face array takes a member through the node-by-node closures and the
+    # launches per level; constant arrays make it the same problem as the
+    # scalar face. The two cycles differ by roundings, so the PCG inside takes
+    # the same number of iterations, or one more or less where a residual meets
+    # its bound within roundings, and both fields meet the residual bound
+    # (their difference: the conditioning bar of this file).
+    def member(dims, arrays):
+        rng = np.random.Generator(np.random.PCG64(sum(dims)))
+        p = GridProblem(*dims, a=-1.0, b=-1.0, az=-1.0)
+        if coef == "divk":
+            p = GridProblem(*dims, coef_kind=abi.COEF_DIVK)
+            p.k = np.exp(0.5 * rng.standard_normal(p.n))
+        p.f = rng.standard_normal(p.n)
+        robin = FaceBC.robin(2.0, 1.0, 0.1)
+        if arrays:
+            robin.alpha_arr = np.full(dims[1] * dims[2], 2.0)
+        p.faces = [robin, FaceBC.dirichlet(0.0), FaceBC.neumann(0.1), FaceBC.dirichlet(0.5), FaceBC.dirichlet(0.0),
+                   FaceBC.neumann(0.0)]
+        return p
+
+    got = []
+    for arrays in (False, True):
+        ms = [member(d, arrays) for d in LOWER]
+        with Batch(ms, bf16_coefficients=bf16, **FIXED) as b:
+            got.append((ms, b.solve(TOL), b.read()))
+    for q in range(len(LOWER)):
+        its = []
+        for ms, reps, fields in got:
+            assert reps[q].converged
+            bb, ax = oracle_mod.rs_folded(ms[q], fields[q])
+            assert np.linalg.norm(bb - ax) / np.linalg.norm(bb) <= 1.01 * TOL
+            its.append(reps[q].iterations)
+        assert abs(its[0] - its[1]) <= 1
+        assert rel_l2(got[0][2][q], got[1][2][q]) <= 1e-7
