@@ -244,6 +244,10 @@ inline dim3 apply_grid(const GridDev& g) { return stencil_grid_auto(g, g.n > (1L
 dim3 fused_grid(const GridDev& g);
 // launch shape of the marching single-pass sweep (64 x 8 interior column tiles, z chunks)
 dim3 march_grid(const GridDev& g);
+// launch shape of the single-pass sweep in registers (30 columns x `rows` rows
+// per block, `resident` blocks per SM), with the z chunks of the least work in
+// whole waves
+dim3 pair_grid(const GridDev& g, int rows, int resident);
 // launch shape of the staged single-pass sweep (32 x 8 column tiles, z chunks
 // for about four resident blocks per SM over two waves)
 dim3 sweep_grid(const GridDev& g);

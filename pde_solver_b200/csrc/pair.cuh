@@ -1,0 +1,273 @@
+// Whole red-black Gauss-Seidel sweep in one pass over memory for large 3D levels
+// with constant coefficients (k_rbgs_pair).
+//
+// Two colour passes (k_rbgs) each read all of x and b and use half of every
+// sector. One sweep needs x and b read once and x written once. A lane
+// owns the columns (i, j0 .. j0 + R - 1) and marches through z two planes per
+// step: at a node of column parity a it updates the first colour on plane
+// P = p + a and the second colour on plane P - 1. Both are the lane's own
+// column, so
+// - the old values of the first colour are never read: one x value per step
+//   and column is loaded (plane P + 1, second colour), the one below is the
+//   previous step's;
+// - a neighbour column has the other parity, so its old value on plane P is its
+//   value below (P - 1 of the neighbour) or above, and its new first-colour
+//   value on plane P - 1 is the one of this step or of the previous one: both
+//   come from the neighbour's registers, by a shuffle in x, from the same lane
+//   in y, through shared memory between the warps of a block (one barrier per
+//   two planes);
+// - every lane works in every step, whatever its colour.
+// Tiles overlap by one column and row on each side, whose first colour is
+// recomputed from old values: blocks never read each other's results, the sweep
+// reads x_in and writes x_out, and is race free and deterministic. The update is
+// that of k_rbgs. x_in's boundary entries are zero, x_out's are not written.
+// ZERO: x_in is identically zero and not read. DOT: as in k_rbgs.
+// DRAM and issue bound: FP32 513^3 421 us per sweep against 737 for two colour
+// passes (1.62 GB, 250 us at the copy rate; about 110 instructions per lane and column
+// step); FP64 257^3 101 against 162, 300^3 139 against 261. With divergence-form
+// coefficients the neighbours' k made it as slow as two passes (230 to 260 us
+// against 226 at 257^3), so those levels keep the colour passes.
+#pragma once
+
+#include "cluster.cuh"
+#include "kernels.cuh"
+
+namespace pdeb {
+
+constexpr int kPairCols = 30;  // columns a warp writes
+// Rows per lane, warps per block and blocks per SM. FP32 at 513^3: 4 x 8 x 2
+// 421 us, 4 x 4 x 5 418 (spills), 3 x 8 x 3 443, 6 x 4 x 3 425, 8 x 4 x 3 501;
+// FP64 at 257^3 / 300^3: 3 x 8 x 2 101 / 139, 2 x 16 x 1 111 / 153, 2 x 8 x 2
+// 107 / 152, 3 x 4 x 4 101 / 154.
+template <int R_, int W_, int B_>
+struct PairShapeOf {
+  static constexpr int R = R_, W = W_, kMinBlocks = B_;
+  static constexpr int kRows = R_ * W_ - 2;  // rows a block writes
+};
+template <typename T>
+using PairShape = std::conditional_t<sizeof(T) == 4, PairShapeOf<4, 8, 2>, PairShapeOf<3, 8, 2>>;
+
+// Closure factors c1 of the six faces (per face, 0 for Dirichlet).
+struct PairFold {
+  double lo[3], hi[3];
+};
+
+// Quotients by one divisor as in RoundedDiv (the general division's bits), the
+// range test on the dividend's magnitude alone: an unsafe divisor makes the
+// range empty.
+template <typename T>
+struct PairDiv {
+  T b, y;
+  __device__ __forceinline__ void init(T d, T& least) {
+    b = d;
+    const T m = fabs(d);
+    if constexpr (sizeof(T) == 4) {
+      y = __frcp_rn(d);
+      if (!(m > 0x1p-40f && m < 0x1p40f) || (__float_as_uint(d) & 0x7fffffu) == 0x7fffffu) least = INFINITY;
+    } else {
+      RoundedDiv q;
+      q.init(d);
+      y = q.y;
+      if (!q.safe) least = INFINITY;
+    }
+  }
+  // for |a| in [least, kMost); 0 where y is
+  __device__ __forceinline__ T operator()(T a) const {
+    if constexpr (sizeof(T) == 4) {
+      float q = __fmul_rn(a, y);
+      q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+      return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+    } else {
+      double q = __dmul_rn(a, y);
+      q = __fma_rn(__fma_rn(-b, q, a), y, q);
+      return __fma_rn(__fma_rn(-b, q, a), y, q);
+    }
+  }
+  static constexpr T kLeast = sizeof(T) == 4 ? T(0x1p-60) : T(0x1p-600);
+  static constexpr T kMost = sizeof(T) == 4 ? T(0x1p60) : T(0x1p600);
+};
+
+template <typename T, bool ZERO, bool DOT, class Post, class S = PairShape<T>>
+__global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
+    k_rbgs_pair(LevelGeo g, PairFold fold, CoefConst cf, const T* __restrict__ b, const T* __restrict__ xin,
+                T* __restrict__ xout, int first, const Ctl* ctl, RedSlot slot, Post post) {
+  if (ctl_skip_dep(ctl)) return;
+  constexpr int R = S::R, W = S::W;
+  constexpr unsigned kAll = 0xffffffffu;
+  __shared__ T ex[2][W][2][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * kPairCols + lane, j0 = blockIdx.y * (W * R - 2) + warp * R;
+  const int len = g.nz - 2, chunk = (len + gridDim.z - 1) / gridDim.z;
+  const int k0 = 1 + blockIdx.z * chunk, k1 = min(g.nz - 1, k0 + chunk);
+  double acc[1] = {0.0};
+  if (k0 < k1) {
+    const int nx = g.nx, ny = g.ny, nz = g.nz, sxy = (int)g.sxy;
+    const int a0 = (i + j0 + k0 - 1 + first) & 1;  // parity of the even rows
+    unsigned inm = 0, outm = 0;
+    unsigned ro[R];  // the node of row r on its plane P, in bytes of T from (0, 0) of plane p; clamped to the grid in x and y
+    const int ic = min(i, nx - 1);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int j = j0 + r, row = warp * R + r;
+      if (i >= 1 && i <= nx - 2 && j >= 1 && j <= ny - 2) {
+        inm |= 1u << r;
+        if (lane >= 1 && lane <= kPairCols && row >= 1 && row <= W * R - 2) outm |= 1u << r;
+      }
+      ro[r] = (unsigned)(min(j, ny - 1) * nx + ic + (((r & 1) ? !a0 : a0) ? sxy : 0)) * (unsigned)sizeof(T);
+    }
+    const unsigned lo = (unsigned)(min(max(j0 - 1, 0), ny - 1) * nx + ic + (a0 ? sxy : 0)) * (unsigned)sizeof(T);
+    const unsigned hi =
+        (unsigned)(min(j0 + R, ny - 1) * nx + ic + ((((R - 1) & 1) ? !a0 : a0) ? sxy : 0)) * (unsigned)sizeof(T);
+    const bool edge = lane == 0 || lane == 31;  // one x neighbour outside the warp
+    const int eo = (lane == 0 ? (ic > 0 ? -1 : 0) : (ic < nx - 1 ? 1 : 0)) * (int)sizeof(T);
+    const T fxl = i == 1 ? T(fold.lo[0]) : T(0), fxh = i == nx - 2 ? T(fold.hi[0]) : T(0);
+    const T fyl = T(fold.lo[1]), fyh = T(fold.hi[1]), fzl = T(fold.lo[2]), fzh = T(fold.hi[2]);
+    int p = k0 - 1;
+
+    T zm[R], vp[R];  // old value on plane P - 1, first colour on plane P - 2
+    struct In {      // what a step reads: x on plane P + 1, b on P and P - 1, neighbours outside the warp on P
+      T zp[R], b1[R], b2[R], xe[R], ylo, yhi;
+    };
+    // loads of the step at q; CL: planes clamped to the grid
+    auto load = [&](In& in, int q, auto clamp) {
+      constexpr bool CL = decltype(clamp)::value;
+      // plane P + d of a row of parity a: its base is the same in all lanes (the
+      // parity is in ro) unless it is clamped
+      auto get = [&](const T* x, int a, int d, unsigned o) -> T {
+        const long long plane = CL ? min(max(q + a + d, 0), nz - 1) - a : q + d;
+        if constexpr (CL) return x[plane * sxy + (long long)(o / (unsigned)sizeof(T))];
+        return *reinterpret_cast<const T*>(reinterpret_cast<const char*>(x + plane * sxy) + o);
+      };
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int a = (r & 1) ? 1 - a0 : a0;
+        in.zp[r] = ZERO ? T(0) : get(xin, a, 1, ro[r]);
+        in.xe[r] = !ZERO && edge ? get(xin, a, 0, ro[r] + eo) : T(0);
+        in.b1[r] = get(b, a, 0, ro[r]);
+        in.b2[r] = get(b, a, -1, ro[r]);
+      }
+      in.ylo = ZERO ? T(0) : get(xin, a0, 0, lo);
+      in.yhi = ZERO ? T(0) : get(xin, ((R - 1) & 1) ? 1 - a0 : a0, 0, hi);
+    };
+    const Stencil<T> st = cf.template at<T, 3>(GridDev{}, 0);
+    PairDiv<T> dv[R];  // by the centre of each row with its x and y closures
+    T least = PairDiv<T>::kLeast;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int a = (r & 1) ? 1 - a0 : a0;
+      zm[r] = ZERO ? T(0)
+                   : xin[(long long)(min(max(p + a - 1, 0), nz - 1) - a) * sxy +
+                         (long long)(ro[r] / (unsigned)sizeof(T))];
+      vp[r] = T(0);
+      T c = st.c;
+      c += st.xm * fxl;
+      c += st.xp * fxh;
+      if (j0 + r == 1) c += st.ym * fyl;
+      if (j0 + r == ny - 2) c += st.yp * fyh;
+      dv[r].init(c, least);
+      if (!(inm >> r & 1)) dv[r].y = T(0);
+    }
+    // numerators to values, with one range test for all rows
+    auto quotients = [&](T (&v)[R]) {
+      bool ok = true;
+#pragma unroll
+      for (int r = 0; r < R; ++r) ok = ok && fabs(v[r]) >= least && fabs(v[r]) < PairDiv<T>::kMost;
+      if (ok) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = dv[r](v[r]);
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = inm >> r & 1 ? v[r] / dv[r].b : T(0);
+      }
+    };
+    // near a z face: the values of interior nodes, centres with the z closures
+    auto edge_quotients = [&](T (&v)[R], int pe, int po) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int P = (r & 1) ? po : pe;
+        T c = dv[r].b;
+        if (P == 1) c += st.zm * fzl;
+        if (P == nz - 2) c += st.zp * fzh;
+        v[r] = (inm >> r & 1) && P >= 1 && P <= nz - 2 ? v[r] / c : T(0);
+      }
+    };
+    int buf = 0;
+    // One step at p. HOT: every node of it is off the z faces and inside the chunk.
+    auto step = [&](const In& in, In& next, auto hot) {
+      constexpr bool HOT = decltype(hot)::value;
+      const int pe = p + a0, po = p + 1 - a0;  // P of the even and odd rows
+      if constexpr (HOT)
+        load(next, p + 2, std::false_type{});
+      else if (p + 2 <= k1)
+        load(next, p + 2, std::true_type{});
+      // node of row r on plane P + d (d = 0, -1), if this block writes it
+      auto put = [&](int d, int r, T val, T rhs) {
+        const int P = ((r & 1) ? po : pe) + d;
+        if ((outm >> r & 1) && (HOT || (P >= k0 && P < k1))) {
+          *reinterpret_cast<T*>(reinterpret_cast<char*>(xout + (long long)(p + d) * sxy) + ro[r]) = val;
+          if constexpr (DOT) acc[0] += double(rhs) * double(val);
+        }
+      };
+      T s[R], v[R], w[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) s[r] = ((r & 1) ? !a0 : a0) ? zm[r] : in.zp[r];  // as the neighbours read it
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        T xl = T(0), xr = T(0), yl = T(0), yh = T(0);
+        if constexpr (!ZERO) {
+          xl = __shfl_up_sync(kAll, s[r], 1);
+          xr = __shfl_down_sync(kAll, s[r], 1);
+          if (lane == 0) xl = in.xe[r];
+          if (lane == 31) xr = in.xe[r];
+          yl = r > 0 ? s[r > 0 ? r - 1 : 0] : in.ylo;
+          yh = r < R - 1 ? s[r < R - 1 ? r + 1 : 0] : in.yhi;
+        }
+        v[r] = in.b1[r] - nb_sum<T>(st, xr, xl, yh, yl, in.zp[r], zm[r], 3);
+      }
+      if constexpr (HOT)
+        quotients(v);
+      else
+        edge_quotients(v, pe, po);
+#pragma unroll
+      for (int r = 0; r < R; ++r) put(0, r, v[r], in.b1[r]);
+#pragma unroll
+      for (int r = 0; r < R; ++r) s[r] = ((r & 1) ? !a0 : a0) ? vp[r] : v[r];
+      ex[buf][warp][0][lane] = s[0];
+      ex[buf][warp][1][lane] = s[R - 1];
+      __syncthreads();
+      const T nlo = ex[buf][warp > 0 ? warp - 1 : 0][1][lane];
+      const T nhi = ex[buf][warp < W - 1 ? warp + 1 : 0][0][lane];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const T xl = __shfl_up_sync(kAll, s[r], 1), xr = __shfl_down_sync(kAll, s[r], 1);
+        const T yl = r > 0 ? s[r > 0 ? r - 1 : 0] : nlo, yh = r < R - 1 ? s[r < R - 1 ? r + 1 : 0] : nhi;
+        w[r] = in.b2[r] - nb_sum<T>(st, xr, xl, yh, yl, v[r], vp[r], 3);
+      }
+      if constexpr (HOT)
+        quotients(w);
+      else
+        edge_quotients(w, pe - 1, po - 1);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        put(-1, r, w[r], in.b2[r]);
+        zm[r] = in.zp[r];
+        vp[r] = v[r];
+      }
+      buf ^= 1;
+      p += 2;
+    };
+    In A, B;
+    load(A, p, std::true_type{});
+    while (p <= k1) {
+      // (hot: the loads of the next step need no clamping either)
+      if (p > k0 && p > 2 && p + 1 < k1 && p + 4 <= nz - 1)
+        step(A, B, std::true_type{});
+      else
+        step(A, B, std::false_type{});
+      A = B;
+    }
+  }
+  if constexpr (DOT) grid_reduce<1, false>(acc, slot, post);
+}
+
+}  // namespace pdeb

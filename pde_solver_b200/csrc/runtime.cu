@@ -169,6 +169,23 @@ dim3 march_grid(const GridDev& g) {
   return dim3(xy.x, xy.y, (unsigned)chunks);
 }
 
+dim3 pair_grid(const GridDev& g, int rows, int resident) {
+  const dim3 xy((g.nx - 2 + 29) / 30, (g.ny - 2 + rows - 1) / rows, 1);
+  const long long xyb = (long long)xy.x * xy.y, wave = 148LL * resident;
+  const int len = g.nz - 2;
+  // the fewest plane steps over all waves; a block takes about 3 planes more than it owns
+  int best = 1;
+  long long cost = -1;
+  for (int z = 1; z == 1 || (len + z - 1) / z >= 16; ++z) {
+    const long long t = (xyb * z + wave - 1) / wave * ((len + z - 1) / z + 3);
+    if (cost < 0 || t < cost) {
+      cost = t;
+      best = z;
+    }
+  }
+  return dim3(xy.x, xy.y, cap_chunks(xyb, best));
+}
+
 dim3 stencil_grid_full(const GridDev& g, int zchunk) {
   const int chunks = (g.nz + zchunk - 1) / zchunk;
   const dim3 xy((g.nx + kBx - 1) / kBx, (g.ny + kBy - 1) / kBy, 1);

@@ -13,6 +13,7 @@
 #include "cluster_vcycle.cuh"
 #include "host.h"
 #include "march.cuh"
+#include "pair.cuh"
 #include "sweep.cuh"
 
 namespace pdeb {
@@ -552,6 +553,7 @@ struct Hierarchy {
     const RestrictTap* rt[3] = {nullptr, nullptr, nullptr};  // restriction onto this level (null: ext factors per node)
     bool single_pass = false;  // sweeps by k_rbgs_sweep (x_in -> x_out) instead of colour passes
     bool march = false;        // sweeps by k_rbgs_march (x_in -> x_out) instead of colour passes
+    bool pair = false;         // sweeps by k_rbgs_pair (between xa and r) instead of colour passes
   };
   // With PDEB200_STAGED_SWEEP set, levels with at least this many nodes use
   // the staged single-pass sweep (FP64 constant or divergence-form
@@ -567,6 +569,13 @@ struct Hierarchy {
   // 226 us per sweep on a box where a colour pass takes 113 us, so the colour
   // passes stay the default.
   static constexpr long long kMarchMinNodes = 1LL << 18;
+  // 3D levels of at least this many nodes with constant coefficients and closure
+  // factors per face smooth with k_rbgs_pair (PDEB200_PAIR_MIN sets the number):
+  // below, two colour passes out of L2 are faster. Convection-diffusion solves,
+  // with it against without: FP32 513^3 70 / 84 ms, 300^3 21.5 / 23.6, 257^3 13.8 /
+  // 14.4, 225^3 11.2 / 10.7; FP64 300^3 24.7 / 26.4, 257^3 16.9 / 17.3, 225^3 12.8 /
+  // 12.8, 171^3 7.8 / 7.1. A plane's byte offsets take 32 bits (sxy < 2^27).
+  static constexpr long long kPairMinNodes = 1LL << 24;
   static constexpr bool kSweepCoef =
       std::is_same<T, double>::value &&
       (std::is_same<Coef, CoefConst>::value || std::is_same<Coef, CoefDivk<double>>::value);
@@ -783,14 +792,26 @@ struct Hierarchy {
                                 ctx->stream));
       PDEB_CUDA(cudaStreamSynchronize(ctx->stream));
     }
+    const char* pair_env = std::getenv("PDEB200_PAIR_MIN");
+    const long long pair_min = pair_env ? std::atoll(pair_env) : kPairMinNodes;
     // result buffer of each level after a V-cycle (fixed, so launches can be captured):
     // the first sweep from zero writes xa, every later sweep flips the buffer
+    ExtCoef pair_ext;
     for (size_t l = 0; l < levels.size(); ++l) {
       Level& L = levels[l];
       L.single_pass = kSweepCoef && sweep_env && !fused && l + 1 < levels.size() && L.g.dim == 3 &&
                       L.g.n >= kSweepMinNodes;
       L.march = kSweepCoef && march_env && !fused && !L.single_pass && l + 1 < levels.size() && L.g.dim == 3 &&
                 L.g.n >= kMarchMinNodes;
+      L.pair = std::is_same<Coef, CoefConst>::value && !fused && !L.single_pass && !L.march && l + 1 < levels.size() &&
+               (int)l != cv_l0 && (int)l != tail_l0 && L.g.dim == 3 && L.g.n >= pair_min && L.g.sxy < (1LL << 27) &&
+               ext_coef(L.g, &pair_ext);
+      if (L.pair) {
+        // the sweeps before the residual end in xa (sweeps_from), those after
+        // the correction go back and forth from there
+        L.out = (post & 1) ? L.r : L.xa;
+        continue;
+      }
       if (!fused && !L.single_pass && !L.march) {
         L.out = L.xa;
         continue;
@@ -815,6 +836,43 @@ struct Hierarchy {
     const dim3 grid = rbgs_grid(L.g), block = stencil_block();
     const dim3 zgrid = stencil_grid_auto(L.g);  // the pass from zero (fewer registers) keeps the default
     const double dofs = interior_dofs(L.g);
+    if constexpr (std::is_same<Coef, CoefConst>::value) {
+      if (L.pair) {
+        const dim3 pgrid = pair_grid(L.g, PairShape<T>::kRows, PairShape<T>::kMinBlocks);
+        const dim3 pblock(32 * PairShape<T>::W);
+        const LevelGeo pg = level_geo(L.g);
+        PairFold pf;
+        {
+          ExtCoef e;
+          ext_coef(L.g, &e);
+          for (int a = 0; a < 3; ++a) {
+            pf.lo[a] = e.lo[a];
+            pf.hi[a] = e.hi[a];
+          }
+        }
+        // from zero: the last sweep ends in xa
+        if (from_zero) cur = (sweeps & 1) ? L.r : L.xa;
+        for (int s = 0; s < sweeps; ++s) {
+          const bool zero = from_zero && s == 0;
+          T* out = cur == L.xa ? L.r : L.xa;
+          const T* in = cur;
+          ProfScope ps(ctx, zero ? "pair_sweep_zero" : "pair_sweep", lvl,
+                       dofs * (zero ? 2.0 : 3.0) * sizeof(T));
+          if (zero)
+            launch_dep(ctx, pgrid, pblock, 0, k_rbgs_pair<T, true, false, NoPost>, pg, pf, L.cf, b, in, out, first,
+                       ctl, RedSlot{}, NoPost{});
+          else if (dot_last && s + 1 == sweeps)
+            launch_dep(ctx, pgrid, pblock, 0, k_rbgs_pair<T, false, true, PostBeta>, pg, pf, L.cf, b, in, out, first,
+                       ctl, *dot_last, PostBeta{const_cast<Ctl*>(ctl)});
+          else
+            launch_dep(ctx, pgrid, pblock, 0, k_rbgs_pair<T, false, false, NoPost>, pg, pf, L.cf, b, in, out, first,
+                       ctl, RedSlot{}, NoPost{});
+          ctx->count();
+          cur = out;
+        }
+        return cur;
+      }
+    }
     if constexpr (kSweepCoef) {
       if (L.march) {
         constexpr size_t smem = march_smem_bytes<Coef>();
@@ -1003,7 +1061,7 @@ struct Hierarchy {
                    gf, gc, e, C.g, (const T*)C.out, cur, ctl);
     }
     ctx->count();
-    if (l == 0 && dot_slot && post > 0 && L.march) {
+    if (l == 0 && dot_slot && post > 0 && (L.march || L.pair)) {
       // the last sweep also sums r.z (b is r on level 0) and forms beta
       cur = sweeps_from(ctx, L, b, cur, post, 1, false, ctl, l, dot_slot);
       dot_done = true;
