@@ -248,6 +248,9 @@ dim3 march_grid(const GridDev& g);
 // per block, `resident` blocks per SM), with the z chunks of the least work in
 // whole waves
 dim3 pair_grid(const GridDev& g, int rows, int resident);
+// launch shape of the column-marching apply (32 columns x `rows` rows x about
+// `planes` planes per block)
+dim3 col_grid(const GridDev& g, int rows, int planes);
 // launch shape of the staged single-pass sweep (32 x 8 column tiles, z chunks
 // for about four resident blocks per SM over two waves)
 dim3 sweep_grid(const GridDev& g);

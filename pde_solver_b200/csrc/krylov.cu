@@ -126,6 +126,8 @@ struct PostBiResid {  // r = b - Ax (true residual) or s - omega t
 template <typename T>
 __global__ void k_bi_p(long long n, T* __restrict__ p, const T* __restrict__ r, const T* __restrict__ v, int first,
                        const Ctl* ctl) {
+  grid_dep_wait();
+  grid_dep_release();
   if (ctl_stopped(ctl)) return;
   const double beta = ctl->beta, omega = ctl->omega;
   for (long long t = gtid(); t < n; t += gstride())
@@ -136,6 +138,8 @@ __global__ void k_bi_p(long long n, T* __restrict__ p, const T* __restrict__ r, 
 template <typename T, class Post>
 __global__ void k_bi_s(long long n, T* __restrict__ s, const T* __restrict__ r, const T* __restrict__ v, RedSlot slot,
                        Post post, const Ctl* ctl) {
+  grid_dep_wait();
+  grid_dep_release();
   if (ctl_stopped(ctl)) return;
   const double alpha = ctl->alpha;
   double acc[1] = {0.0};
@@ -150,11 +154,15 @@ __global__ void k_bi_s(long long n, T* __restrict__ s, const T* __restrict__ r, 
 // early exit of the s-check: x += alpha p, then done
 template <typename T>
 __global__ void k_bi_exit(long long n, T* __restrict__ x, const T* __restrict__ p, Ctl* ctl) {
+  grid_dep_wait();
+  grid_dep_release();
   if (ctl->done || !ctl->stop || ctl->aux[1] == 0.0) return;
   const double alpha = ctl->alpha;
   for (long long t = gtid(); t < n; t += gstride()) x[t] = T(double(x[t]) + alpha * double(p[t]));
 }
 __global__ void k_bi_exit_flag(Ctl* ctl) {
+  grid_dep_wait();
+  grid_dep_release();
   if (ctl->done || !ctl->stop || ctl->aux[1] == 0.0) return;
   ctl->iter += 1;
   ctl->done = 1;
@@ -165,31 +173,48 @@ __global__ void k_bi_exit_flag(Ctl* ctl) {
 template <typename T>
 __global__ void k_bi_x(long long n, T* __restrict__ x, const T* __restrict__ p, const T* __restrict__ s,
                        const Ctl* ctl) {
+  grid_dep_wait();
+  grid_dep_release();
   if (ctl_stopped(ctl)) return;
   const double alpha = ctl->alpha, omega = ctl->omega;
   for (long long t = gtid(); t < n; t += gstride())
     x[t] = T(double(x[t]) + alpha * double(p[t]) + omega * double(s[t]));
 }
 
-// r = s - omega t, sum r^2 (recursive residual of the preconditioned form)
+// r = s - omega t, sums r^2 and rhat.r (recursive residual and the next rho of
+// the preconditioned form)
 template <typename T, class Post>
 __global__ void k_bi_r(long long n, T* __restrict__ r, const T* __restrict__ s, const T* __restrict__ t_,
-                       RedSlot slot, Post post, const Ctl* ctl) {
+                       const T* __restrict__ rhat, RedSlot slot, Post post, const Ctl* ctl) {
+  grid_dep_wait();
+  grid_dep_release();
   if (ctl_stopped(ctl)) return;
   const double omega = ctl->omega;
-  double acc[1] = {0.0};
+  double acc[2] = {0.0, 0.0};
   for (long long t = gtid(); t < n; t += gstride()) {
     const T rv = T(double(s[t]) - omega * double(t_[t]));
     r[t] = rv;
     acc[0] += double(rv) * double(rv);
+    acc[1] += double(rhat[t]) * double(rv);
   }
-  grid_reduce<1, false>(acc, slot, post);
+  grid_reduce<2, false>(acc, slot, post);
 }
+
+// PostBiResid, and the rho of the next iteration
+struct PostBiResidRho {
+  Ctl* c;
+  __device__ void operator()(const double* v) const {
+    PostBiResid{c, 1}(v);
+    if (!c->done) PostBiRho{c}(v + 1);
+  }
+};
 
 // two dots in one pass: {t.t, t.s}
 template <typename T, class Post>
 __global__ void k_dot_tt_ts(long long n, const T* __restrict__ t_, const T* __restrict__ s, RedSlot slot, Post post,
                             const Ctl* ctl) {
+  grid_dep_wait();
+  grid_dep_release();
   if (ctl_stopped(ctl)) return;
   double acc[2] = {0.0, 0.0};
   for (long long t = gtid(); t < n; t += gstride()) {
@@ -220,9 +245,20 @@ struct PostBiInit {  // |r0| check and rho_prev = alpha = omega = 1
   }
 };
 
+// PostBiInit, and the first rho: rhat = r, so it is |r|^2
+struct PostBiInitRho {
+  Ctl* c;
+  __device__ void operator()(const double* v) const {
+    PostBiInit{c, 1}(v);
+    if (!c->done) PostBiRho{c}(v);
+  }
+};
+
 template <typename T, class Post>
 __global__ void k_dot_skip(long long n, const T* __restrict__ a, const T* __restrict__ b, RedSlot slot, Post post,
                            const Ctl* ctl) {
+  grid_dep_wait();
+  grid_dep_release();
   if (ctl_stopped(ctl)) return;
   double acc[1] = {0.0};
   for (long long t = gtid(); t < n; t += gstride()) acc[0] += double(a[t]) * double(b[t]);
@@ -550,49 +586,87 @@ pdeb200_status gmres_reference(Context* ctx, DevProblem& P, const Coef& cf, cons
 //   p = r + beta(p - omega v); phat = M p; v = A phat; alpha = rho/(rhat.v)
 //   s = r - alpha v; shat = M s; t = A shat; omega = (t.s)/(t.t)
 //   x += alpha phat + omega shat; r = s - omega t   (relative rule on |r|)
+// One object serves every outer step of a refinement, as MgPcgCore does. rhat is
+// b itself, phat the buffer that the first V-cycle of an iteration writes, and
+// the dot products come from the kernels that produce their operands where the
+// finest level allows it (k_apply_columns): 513^3 FP32 moved 26 vectors per
+// iteration besides the V-cycles, now 21.
 template <class Coef, class HierT, typename T>
-pdeb200_status mg_bicgstab_core(Context* ctx, HierT& H, const GridDev& g, const Coef& cf, const T* b, T* x,
-                                int max_iter, double tol, const pdeb200_options* o, int* iters) {
-  const long long n = g.n;
-  Buf buf(sizeof(T) * n * 7, ctx->stream);
-  T* B = buf.template as<T>();
-  T *r = B, *rhat = B + n, *p = B + 2 * n, *v = B + 3 * n, *s = B + 4 * n, *t = B + 5 * n, *ph = B + 6 * n;
-  PDEB_CUDA(cudaMemsetAsync(B, 0, sizeof(T) * n * 7, ctx->stream));
-  PDEB_CUDA(cudaMemsetAsync(x, 0, sizeof(T) * n, ctx->stream));
-  PDEB_CUDA(cudaMemcpyAsync(r, b, sizeof(T) * n, cudaMemcpyDeviceToDevice, ctx->stream));
-  PDEB_CUDA(cudaMemcpyAsync(rhat, b, sizeof(T) * n, cudaMemcpyDeviceToDevice, ctx->stream));
-  ctl_init(ctx, max_iter, tol, 1e-300);
-  Ctl* C = ctx->d_ctl;
-  const int nb = vec_blocks(n, ctx);
-  k_dot<T, PostBiInit><<<nb, 256, 0, ctx->stream>>>(n, r, r, ctx->slot(), PostBiInit{C, 1}, nullptr);
-  ctx->count();
-  const dim3 grid = stencil_grid_auto(g), block = stencil_block();
-  T* z = H.z();
-  auto iterate = [&](int it) {
-    k_dot_skip<T, PostBiRho><<<nb, 256, 0, ctx->stream>>>(n, rhat, r, ctx->slot(), PostBiRho{C}, C);
-    k_bi_p<T><<<nb, 256, 0, ctx->stream>>>(n, p, r, v, it == 0, C);
-    H.vcycle(ctx, p, C);
-    PDEB_CUDA(cudaMemcpyAsync(ph, z, sizeof(T) * n, cudaMemcpyDeviceToDevice, ctx->stream));
-    k_apply_folded<Coef, T, 0, NoPost><<<grid, block, 0, ctx->stream>>>(g, cf, ph, v, RedSlot{}, NoPost{}, C);
-    k_dot_skip<T, PostBiAlpha><<<nb, 256, 0, ctx->stream>>>(n, rhat, v, ctx->slot(), PostBiAlpha{C}, C);
-    k_bi_s<T, PostBiS><<<nb, 256, 0, ctx->stream>>>(n, s, r, v, ctx->slot(), PostBiS{C, 1}, C);
-    k_bi_exit<T><<<nb, 256, 0, ctx->stream>>>(n, x, ph, C);
-    k_bi_exit_flag<<<1, 1, 0, ctx->stream>>>(C);
-    H.vcycle(ctx, s, C);
-    k_apply_folded<Coef, T, 0, NoPost><<<grid, block, 0, ctx->stream>>>(g, cf, z, t, RedSlot{}, NoPost{}, C);
-    k_dot_tt_ts<T, PostBiOmega><<<nb, 256, 0, ctx->stream>>>(n, t, s, ctx->slot(), PostBiOmega{C}, C);
-    k_bi_x<T><<<nb, 256, 0, ctx->stream>>>(n, x, ph, z, C);
-    k_bi_r<T, PostBiResid><<<nb, 256, 0, ctx->stream>>>(n, r, s, t, ctx->slot(), PostBiResid{C, 1}, C);
-    ctx->count(12);
-  };
-  // iterations after the first are identical
+struct MgBicgCore {
+  Buf buf;
   StepGraph graph;
-  auto step = [&](int it) { graph.step(ctx, n, it, iterate, [&](int) { iterate(1); }); };
-  pdeb200_status st = drive(ctx, o, max_iter + 1, step, false);
-  const Ctl c = ctl_poll(ctx);
-  *iters = c.iter;
-  return st;
-}
+
+  pdeb200_status run(Context* ctx, HierT& H, const GridDev& g, const Coef& cf, const T* b, T* x, int max_iter,
+                     double tol, const pdeb200_options* o, int* iters) {
+    const long long n = g.n;
+    const bool made = buf.bytes() != 0;
+    if (!made) buf = Buf(sizeof(T) * n * 6, ctx->stream);
+    T* B = buf.template as<T>();
+    T *r = B, *p = B + n, *s = B + 2 * n, *v = B + 3 * n, *t = B + 4 * n, *ph = B + 5 * n;
+    // v, t and phat are written on the interior only
+    if (!made) PDEB_CUDA(cudaMemsetAsync(v, 0, sizeof(T) * n * 3, ctx->stream));
+    PDEB_CUDA(cudaMemsetAsync(x, 0, sizeof(T) * n, ctx->stream));
+    PDEB_CUDA(cudaMemcpyAsync(r, b, sizeof(T) * n, cudaMemcpyDeviceToDevice, ctx->stream));
+    const T* rhat = b;
+    ctl_init(ctx, max_iter, tol, 1e-300);
+    Ctl* C = ctx->d_ctl;
+    const int nb = vec_blocks(n, ctx);
+    k_dot<T, PostBiInitRho><<<nb, 256, 0, ctx->stream>>>(n, b, b, ctx->slot(), PostBiInitRho{C}, nullptr);
+    ctx->count();
+    const dim3 grid = stencil_grid_auto(g), block = stencil_block(), vg(nb), vb(256);
+    // y = A q with its sum(s), in one launch or two
+    auto apply = [&](const T* q, const T* w, T* y, auto mode) {
+      constexpr int MODE = decltype(mode)::value;
+      using Post = std::conditional_t<MODE == 1, PostBiAlpha, PostBiOmega>;
+      if constexpr (std::is_same<Coef, CoefConst>::value) {
+        if (H.levels[0].pair) {
+          launch_dep(ctx, col_grid(g, kColW * kColRows, kColPlanesSum), dim3(32 * kColW), 0,
+                     k_apply_columns<T, MODE, Post>, level_geo(g), pair_fold(g), cf, q, w, y, (const Ctl*)C,
+                     ctx->slot(), Post{C});
+          ctx->count();
+          return;
+        }
+      }
+      launch_dep(ctx, grid, block, 0, k_apply_folded<Coef, T, 0, NoPost>, g, cf, q, y, RedSlot{}, NoPost{},
+                 (const Ctl*)C);
+      if constexpr (MODE == 1)
+        launch_dep(ctx, vg, vb, 0, k_dot_skip<T, Post>, n, w, (const T*)y, ctx->slot(), Post{C}, (const Ctl*)C);
+      else
+        launch_dep(ctx, vg, vb, 0, k_dot_tt_ts<T, Post>, n, (const T*)y, w, ctx->slot(), Post{C}, (const Ctl*)C);
+      ctx->count(2);
+    };
+    T* const z = H.z();
+    const bool swap = H.output_swappable();
+    auto iterate = [&](int it) {
+      launch_dep(ctx, vg, vb, 0, k_bi_p<T>, n, p, (const T*)r, (const T*)v, it == 0 ? 1 : 0, (const Ctl*)C);
+      if (swap) {
+        H.set_output(ph);
+        H.vcycle(ctx, p, C);
+        H.set_output(z);
+      } else {
+        H.vcycle(ctx, p, C);
+        PDEB_CUDA(cudaMemcpyAsync(ph, z, sizeof(T) * n, cudaMemcpyDeviceToDevice, ctx->stream));
+      }
+      apply(ph, rhat, v, std::integral_constant<int, 1>{});
+      launch_dep(ctx, vg, vb, 0, k_bi_s<T, PostBiS>, n, s, (const T*)r, (const T*)v, ctx->slot(), PostBiS{C, 1},
+                 (const Ctl*)C);
+      launch_dep(ctx, vg, vb, 0, k_bi_exit<T>, n, x, (const T*)ph, C);
+      launch_dep(ctx, dim3(1), dim3(1), 0, k_bi_exit_flag, C);
+      H.vcycle(ctx, s, C);
+      apply(z, s, t, std::integral_constant<int, 2>{});
+      launch_dep(ctx, vg, vb, 0, k_bi_x<T>, n, x, (const T*)ph, (const T*)z, (const Ctl*)C);
+      launch_dep(ctx, vg, vb, 0, k_bi_r<T, PostBiResidRho>, n, r, (const T*)s, (const T*)t, rhat, ctx->slot(),
+                 PostBiResidRho{C}, (const Ctl*)C);
+      ctx->count(6);
+    };
+    // iterations after the first are identical
+    auto step = [&](int it) { graph.step(ctx, n, it, iterate, [&](int) { iterate(1); }); };
+    pdeb200_status st = drive(ctx, o, max_iter + 1, step, false);
+    const Ctl c = ctl_poll(ctx);
+    *iters = c.iter;
+    return st;
+  }
+};
 
 template <class Coef>
 pdeb200_status mg_bicgstab(Context* ctx, DevProblem& P, const Coef& cf, const pdeb200_problem* hp,
@@ -605,8 +679,8 @@ pdeb200_status mg_bicgstab(Context* ctx, DevProblem& P, const Coef& cf, const pd
   double *bf = bfb.as<double>(), *r = rb.as<double>();
   build_folded_rhs(ctx, P, cf, bf);
   int it = 0;
-  pdeb200_status st = mg_bicgstab_core<Coef, Hierarchy<Coef, double>, double>(
-      ctx, H, P.g, cf, bf, d_x, o->max_iter > 1 ? o->max_iter : 1, o->tol, o, &it);
+  MgBicgCore<Coef, Hierarchy<Coef, double>, double> core;
+  pdeb200_status st = core.run(ctx, H, P.g, cf, bf, d_x, o->max_iter > 1 ? o->max_iter : 1, o->tol, o, &it);
   if (rep) {
     rep->iterations = it;
     rep->converged = st == PDEB200_OK;
@@ -768,6 +842,7 @@ pdeb200_status mixed_refinement(Context* ctx, DevProblem& P, const Coef& cf, con
     auto run = [&](auto& H) {
       using HT = std::decay_t<decltype(H)>;
       MgPcgCore<typename L::F32, HT, float> pcg;
+      MgBicgCore<typename L::F32, HT, float> bicg;
       for (outer = 0; outer < max_outer; ++outer) {
         k_residual_folded<Coef, double, double, 1, PostRRtoAux><<<grid, block, 0, ctx->stream>>>(
             g, cf, d_x, bf, r, ctx->slot(), PostRRtoAux{C}, nullptr);
@@ -793,8 +868,7 @@ pdeb200_status mixed_refinement(Context* ctx, DevProblem& P, const Coef& cf, con
         // 4 of margin covers the FP32 operator's rounding)
         const double step_tol = std::max(io.tol, std::min(0.1, 0.25 * o->tol / rel));
         if (nonsym)
-          is = mg_bicgstab_core<typename L::F32, HT, float>(ctx, H, g, cf32, r32, e32, io.max_iter, step_tol, &io,
-                                                            &it);
+          is = bicg.run(ctx, H, g, cf32, r32, e32, io.max_iter, step_tol, &io, &it);
         else
           is = pcg.run(ctx, H, g, cf32, r32, e32, io.max_iter, step_tol, &io, &it);
         total_inner += it;

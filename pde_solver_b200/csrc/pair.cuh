@@ -104,7 +104,8 @@ __global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
     const int nx = g.nx, ny = g.ny, nz = g.nz, sxy = (int)g.sxy;
     const int a0 = (i + j0 + k0 - 1 + first) & 1;  // parity of the even rows
     unsigned inm = 0, outm = 0;
-    unsigned ro[R];  // the node of row r on its plane P, in bytes of T from (0, 0) of plane p; clamped to the grid in x and y
+    // the node of row r on its plane P, in bytes of T from (0, 0) of plane p; clamped to the grid in x and y
+    unsigned ro[R];
     const int ic = min(i, nx - 1);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -268,6 +269,129 @@ __global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
     }
   }
   if constexpr (DOT) grid_reduce<1, false>(acc, slot, post);
+}
+
+// y = A_fold x of the same levels (MODE 0), with the sum of w y (MODE 1) or the
+// sums of y y and y w (MODE 2), or y = w - A_fold x (MODE 3). A lane marches R
+// rows of a column: each x value is loaded once (plus the rows and columns
+// around a warp), neighbours in x by shuffles, in y and z from registers; the
+// planes two ahead are in flight. FP32 513^3: 238 us (297 by k_apply_folded,
+// 165 at the copy rate), residual 305 (371, 250); with the sums 380, where the
+// separate dot products take another 130 to 165. FP64 300^3: 95 (111), residual no
+// faster (121, 120), so that keeps k_residual_folded.
+constexpr int kColW = 4, kColRows = 4;
+// planes per block: without a sum short chunks spread the work, with one fewer
+// blocks leave fewer partial sums (513^3 FP32 21 / 43 / 86 planes: apply 238 / 242 /
+// 263 us, with a sum 415 / 378 / 387)
+constexpr int kColPlanes = 21, kColPlanesSum = 48;
+inline PairFold pair_fold(const GridDev& g) {
+  ExtCoef e;
+  ext_coef(g, &e);
+  PairFold f;
+  for (int a = 0; a < 3; ++a) {
+    f.lo[a] = e.lo[a];
+    f.hi[a] = e.hi[a];
+  }
+  return f;
+}
+template <typename T, int MODE, class Post, int R = kColRows>
+__global__ void __launch_bounds__(32 * kColW) k_apply_columns(LevelGeo g, PairFold fold, CoefConst cf,
+                                                              const T* __restrict__ x, const T* __restrict__ w,
+                                                              T* __restrict__ y, const Ctl* ctl, RedSlot slot,
+                                                              Post post) {
+  if (ctl_skip_dep(ctl)) return;
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int NV = MODE == 1 ? 1 : (MODE == 2 ? 2 : 0);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = 1 + blockIdx.x * 32 + lane, j0 = 1 + (blockIdx.y * kColW + warp) * R;
+  const int len = g.nz - 2, chunk = (len + gridDim.z - 1) / gridDim.z;
+  const int k0 = 1 + blockIdx.z * chunk, k1 = min(g.nz - 1, k0 + chunk);
+  double acc[NV > 0 ? NV : 1] = {};
+  if (k0 < k1 && j0 <= g.ny - 2) {
+    const int nx = g.nx, ny = g.ny, nz = g.nz, sxy = (int)g.sxy;
+    const int ic = min(i, nx - 1);
+    const bool edge = lane == 0 || lane == 31;
+    const int eo = (lane == 0 ? -1 : (ic < nx - 1 ? 1 : 0)) * (int)sizeof(T);
+    const Stencil<T> st = cf.template at<T, 3>(GridDev{}, 0);
+    unsigned outm = 0, ro[R];  // bytes from (0, 0) of a plane, clamped to the grid
+    T cr[R];                   // centres with the x and y closures
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int j = j0 + r;
+      if (i <= nx - 2 && j <= ny - 2) outm |= 1u << r;
+      ro[r] = (unsigned)(min(j, ny - 1) * nx + ic) * (unsigned)sizeof(T);
+      T c = st.c;
+      c += st.xm * (i == 1 ? T(fold.lo[0]) : T(0));
+      c += st.xp * (i == nx - 2 ? T(fold.hi[0]) : T(0));
+      if (j == 1) c += st.ym * T(fold.lo[1]);
+      if (j == ny - 2) c += st.yp * T(fold.hi[1]);
+      cr[r] = c;
+    }
+    const unsigned lo = (unsigned)((j0 - 1) * nx + ic) * (unsigned)sizeof(T);
+    const unsigned hi = (unsigned)(min(j0 + R, ny - 1) * nx + ic) * (unsigned)sizeof(T);
+    auto get = [&](const T* a, int plane, unsigned o) -> T {
+      return *reinterpret_cast<const T*>(reinterpret_cast<const char*>(a + (long long)plane * sxy) + o);
+    };
+    T zm[R], zc[R], zp[R], zn[R];            // planes k - 1 .. k + 2
+    T xe[R], wv[R], ylo, yhi;                // of plane k, loaded one step before
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      zm[r] = get(x, k0 - 1, ro[r]);
+      zc[r] = get(x, k0, ro[r]);
+      zp[r] = get(x, k0 + 1, ro[r]);
+      xe[r] = edge ? get(x, k0, ro[r] + eo) : T(0);
+      wv[r] = MODE ? get(w, k0, ro[r]) : T(0);
+    }
+    ylo = get(x, k0, lo);
+    yhi = get(x, k0, hi);
+    for (int k = k0; k < k1; ++k) {
+      T xen[R], wn[R], ylon, yhin;
+      const int k2 = min(k + 2, nz - 1);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        zn[r] = get(x, k2, ro[r]);
+        xen[r] = edge ? get(x, k + 1, ro[r] + eo) : T(0);
+        wn[r] = MODE ? get(w, k + 1, ro[r]) : T(0);
+      }
+      ylon = get(x, k + 1, lo);
+      yhin = get(x, k + 1, hi);
+      const bool zed = k == 1 || k == nz - 2;
+      T* const yk = y + (long long)k * sxy;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        T xl = __shfl_up_sync(kAll, zc[r], 1), xr = __shfl_down_sync(kAll, zc[r], 1);
+        if (lane == 0) xl = xe[r];
+        if (lane == 31) xr = xe[r];
+        T c = cr[r];
+        if (zed) {
+          if (k == 1) c += st.zm * T(fold.lo[2]);
+          if (k == nz - 2) c += st.zp * T(fold.hi[2]);
+        }
+        const T yl = r > 0 ? zc[r > 0 ? r - 1 : 0] : ylo, yh = r < R - 1 ? zc[r < R - 1 ? r + 1 : 0] : yhi;
+        T v = c * zc[r] + nb_sum<T>(st, xr, xl, yh, yl, zp[r], zm[r], 3);
+        if (MODE == 3) v = wv[r] - v;
+        if (outm >> r & 1) {
+          *reinterpret_cast<T*>(reinterpret_cast<char*>(yk) + ro[r]) = v;
+          if constexpr (MODE == 1) acc[0] += double(wv[r]) * double(v);
+          if constexpr (MODE == 2) {
+            acc[0] += double(v) * double(v);
+            acc[NV - 1] += double(v) * double(wv[r]);
+          }
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        zm[r] = zc[r];
+        zc[r] = zp[r];
+        zp[r] = zn[r];
+        xe[r] = xen[r];
+        wv[r] = wn[r];
+      }
+      ylo = ylon;
+      yhi = yhin;
+    }
+  }
+  if constexpr (NV > 0) grid_reduce<NV, false>(acc, slot, post);
 }
 
 }  // namespace pdeb

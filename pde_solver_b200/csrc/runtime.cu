@@ -186,6 +186,11 @@ dim3 pair_grid(const GridDev& g, int rows, int resident) {
   return dim3(xy.x, xy.y, cap_chunks(xyb, best));
 }
 
+dim3 col_grid(const GridDev& g, int rows, int planes) {
+  const dim3 xy((g.nx - 2 + 31) / 32, (g.ny - 2 + rows - 1) / rows, 1);
+  return dim3(xy.x, xy.y, cap_chunks((long long)xy.x * xy.y, (g.nz - 2 + planes - 1) / planes));
+}
+
 dim3 stencil_grid_full(const GridDev& g, int zchunk) {
   const int chunks = (g.nz + zchunk - 1) / zchunk;
   const dim3 xy((g.nx + kBx - 1) / kBx, (g.ny + kBy - 1) / kBy, 1);

@@ -841,15 +841,7 @@ struct Hierarchy {
         const dim3 pgrid = pair_grid(L.g, PairShape<T>::kRows, PairShape<T>::kMinBlocks);
         const dim3 pblock(32 * PairShape<T>::W);
         const LevelGeo pg = level_geo(L.g);
-        PairFold pf;
-        {
-          ExtCoef e;
-          ext_coef(L.g, &e);
-          for (int a = 0; a < 3; ++a) {
-            pf.lo[a] = e.lo[a];
-            pf.hi[a] = e.hi[a];
-          }
-        }
+        const PairFold pf = pair_fold(L.g);
         // from zero: the last sweep ends in xa
         if (from_zero) cur = (sweeps & 1) ? L.r : L.xa;
         for (int s = 0; s < sweeps; ++s) {
@@ -1015,9 +1007,19 @@ struct Hierarchy {
       // launch in a replayed graph; 129^3 unchanged); larger levels 148 x 24
       // (12 z chunks at 257^3, an even number of planes per chunk for the
       // two-plane trips: 108.7 -> 103.6 us per launch in the solve)
-      launch_dep(ctx, stencil_grid_auto(L.g, L.g.n > (1LL << 22) ? 148 * 24 : 148 * 6), stencil_block(), 0,
-                 k_residual_folded<Coef, T, T, 0, NoPost>, L.g, L.cf, (const T*)cur, b, L.r, RedSlot{}, NoPost{},
-                 ctl);
+      bool done = false;
+      if constexpr (std::is_same<Coef, CoefConst>::value && sizeof(T) == 4) {
+        if (L.pair) {
+          launch_dep(ctx, col_grid(L.g, kColW * kColRows, kColPlanes), dim3(32 * kColW), 0,
+                     k_apply_columns<T, 3, NoPost>, level_geo(L.g), pair_fold(L.g), L.cf, (const T*)cur, b, L.r, ctl,
+                     RedSlot{}, NoPost{});
+          done = true;
+        }
+      }
+      if (!done)
+        launch_dep(ctx, stencil_grid_auto(L.g, L.g.n > (1LL << 22) ? 148 * 24 : 148 * 6), stencil_block(), 0,
+                   k_residual_folded<Coef, T, T, 0, NoPost>, L.g, L.cf, (const T*)cur, b, L.r, RedSlot{}, NoPost{},
+                   ctl);
     }
     Level& C = levels[l + 1];
     {
@@ -1104,6 +1106,10 @@ struct Hierarchy {
   const RedSlot* dot_slot = nullptr;
   bool dot_done = false;
   T* z() const { return levels[0].out; }
+  // The V-cycle can write its result to another buffer with a zero boundary
+  // (not where a form ends in its second buffer or the tail's table holds xa).
+  bool output_swappable() const { return levels[0].out == levels[0].xa && tail_l0 != 0; }
+  void set_output(T* z) { levels[0].xa = levels[0].out = z; }
 };
 
 // -------------------------------------------------- drivers in other units

@@ -64,3 +64,30 @@ def test_one_pass_in_mixed_precision(monkeypatch, dims):
     assert ra.status == abi.OK and ra.rel_residual <= 1e-11
     assert abs(ra.iterations - rb.iterations) <= 1
     assert np.linalg.norm(a - b) <= 1e-8 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("dims", DIMS[:5])
+@pytest.mark.parametrize("sweeps", [(2, 2), (1, 1)])
+def test_bicgstab_on_column_kernels(monkeypatch, dims, sweeps):
+    # MG-BiCGStab with the apply and its sums in one launch (k_apply_columns,
+    # 32 x 16 columns) against separate ones, in both output buffers of the
+    # V-cycle: two iterations, whose scalars amplify the roundings of differently
+    # ordered sums by up to 1e5: 1e-9 relative
+    p = make(dims)
+    p.c, p.d, p.dz = 3.0, -2.0, 1.0
+    opt = default_options(method=abi.MG_BICGSTAB, tol=0.0, tol_mode=abi.TOL_RELATIVE, max_iter=2,
+                          mg_pre_smooth=sweeps[0], mg_post_smooth=sweeps[1])
+    a, b, ra, rb = both(monkeypatch, p, opt)
+    assert ra.iterations == rb.iterations
+    assert np.linalg.norm(a - b) <= 1e-9 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("dims", DIMS[:5])
+def test_bicgstab_in_mixed_precision_on_column_kernels(monkeypatch, dims):
+    p = make(dims)
+    p.c, p.d, p.dz = 3.0, -2.0, 1.0
+    opt = default_options(method=abi.MG_BICGSTAB, tol=1e-10, tol_mode=abi.TOL_RELATIVE, max_iter=200,
+                          precision=abi.MIXED)
+    a, b, ra, rb = both(monkeypatch, p, opt)
+    assert ra.status == abi.OK and ra.rel_residual <= 1e-10
+    assert np.linalg.norm(a - b) <= 1e-8 * np.linalg.norm(b)  # the bar of the mixed form
