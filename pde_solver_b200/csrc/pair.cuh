@@ -1,8 +1,8 @@
 // Whole red-black Gauss-Seidel sweep in one pass over memory for large 3D levels
-// with constant coefficients (k_rbgs_pair).
+// (k_rbgs_pair), and the apply of the same levels by columns (k_apply_columns).
 //
-// Two colour passes (k_rbgs) each read all of x and b and use half of every
-// sector. One sweep needs x and b read once and x written once. A lane
+// Two colour passes (k_rbgs) each read all of x, b and k and use half of every
+// sector. One sweep needs them read once and x written once. A lane
 // owns the columns (i, j0 .. j0 + R - 1) and marches through z two planes per
 // step: at a node of column parity a it updates the first colour on plane
 // P = p + a and the second colour on plane P - 1. Both are the lane's own
@@ -22,11 +22,13 @@
 // reads x_in and writes x_out, and is race free and deterministic. The update is
 // that of k_rbgs. x_in's boundary entries are zero, x_out's are not written.
 // ZERO: x_in is identically zero and not read. DOT: as in k_rbgs.
-// DRAM and issue bound: FP32 513^3 421 us per sweep against 737 for two colour
-// passes (1.62 GB, 250 us at the copy rate; about 110 instructions per lane and column
-// step); FP64 257^3 101 against 162, 300^3 139 against 261. With divergence-form
-// coefficients the neighbours' k made it as slow as two passes (230 to 260 us
-// against 226 at 257^3), so those levels keep the colour passes.
+// Issue bound (about 110 instructions per lane and column step, 63% of the
+// issue slots), then DRAM: FP32 513^3 421 us per sweep against 737 for two colour
+// passes (250 at the copy rate); FP64 257^3 101 against 162, 300^3 139 against 261.
+// Divergence form: k of the neighbours by shuffles too; FP64 257^3 177 us against
+// 226, BF16 k in FP32 125 against 141. Lanes off the interior keep ordinary
+// dividends: zeros take the division's slow branch and held whole blocks up (258
+// instead of 177).
 #pragma once
 
 #include "cluster.cuh"
@@ -38,14 +40,36 @@ constexpr int kPairCols = 30;  // columns a warp writes
 // Rows per lane, warps per block and blocks per SM. FP32 at 513^3: 4 x 8 x 2
 // 421 us, 4 x 4 x 5 418 (spills), 3 x 8 x 3 443, 6 x 4 x 3 425, 8 x 4 x 3 501;
 // FP64 at 257^3 / 300^3: 3 x 8 x 2 101 / 139, 2 x 16 x 1 111 / 153, 2 x 8 x 2
-// 107 / 152, 3 x 4 x 4 101 / 154.
+// 107 / 152, 3 x 4 x 4 101 / 154. Divergence form FP64 at 257^3: 3 x 8 x 1 177, 2 x 8 x
+// 2 209 (spills), 4 x 4 x 2 183, 3 x 4 x 3 205, 4 x 8 x 1 195.
 template <int R_, int W_, int B_>
 struct PairShapeOf {
   static constexpr int R = R_, W = W_, kMinBlocks = B_;
   static constexpr int kRows = R_ * W_ - 2;  // rows a block writes
 };
-template <typename T>
-using PairShape = std::conditional_t<sizeof(T) == 4, PairShapeOf<4, 8, 2>, PairShapeOf<3, 8, 2>>;
+template <class Coef, typename T>
+using PairShape =
+    std::conditional_t<sizeof(T) == 4, PairShapeOf<4, 8, 2>,
+                       std::conditional_t<std::is_same<Coef, CoefConst>::value, PairShapeOf<3, 8, 2>, PairShapeOf<3, 8, 1>>>;
+
+// k of divergence-form coefficients
+template <class Coef>
+struct PairK {
+  static constexpr bool kHas = false, kOk = std::is_same<Coef, CoefConst>::value;
+  __device__ static const float* field(const Coef&) { return nullptr; }
+};
+template <typename KT>
+struct PairK<CoefDivk<KT>> {
+  static constexpr bool kHas = true, kOk = true;
+  __device__ static const KT* field(const CoefDivk<KT>& c) { return c.k; }
+};
+template <typename T, typename KT>
+__device__ __forceinline__ T pair_k(KT k) {
+  if constexpr (std::is_same<KT, __nv_bfloat16>::value)
+    return T(__bfloat162float(k));
+  else
+    return T(k);
+}
 
 // Closure factors c1 of the six faces (per face, 0 for Dirichlet).
 struct PairFold {
@@ -87,12 +111,16 @@ struct PairDiv {
   static constexpr T kMost = sizeof(T) == 4 ? T(0x1p60) : T(0x1p600);
 };
 
-template <typename T, bool ZERO, bool DOT, class Post, class S = PairShape<T>>
+template <class Coef, typename T, bool ZERO, bool DOT, class Post, class S = PairShape<Coef, T>>
 __global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
-    k_rbgs_pair(LevelGeo g, PairFold fold, CoefConst cf, const T* __restrict__ b, const T* __restrict__ xin,
+    k_rbgs_pair(LevelGeo g, PairFold fold, Coef cf, const T* __restrict__ b, const T* __restrict__ xin,
                 T* __restrict__ xout, int first, const Ctl* ctl, RedSlot slot, Post post) {
   if (ctl_skip_dep(ctl)) return;
   constexpr int R = S::R, W = S::W;
+  constexpr bool kK = PairK<Coef>::kHas;
+  constexpr int RK = kK ? R : 1;
+  const auto* const kf = PairK<Coef>::field(cf);
+  using KT = std::remove_cv_t<std::remove_pointer_t<decltype(kf)>>;
   constexpr unsigned kAll = 0xffffffffu;
   __shared__ T ex[2][W][2][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -128,7 +156,9 @@ __global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
     T zm[R], vp[R];  // old value on plane P - 1, first colour on plane P - 2
     struct In {      // what a step reads: x on plane P + 1, b on P and P - 1, neighbours outside the warp on P
       T zp[R], b1[R], b2[R], xe[R], ylo, yhi;
+      T kc[RK], kp[RK], ke[RK], kl[2], kh[2];  // k on P and P + 1; outside the warp on P (in y also on P - 1)
     };
+    T km[RK], kb[RK];  // k on planes P - 2, P - 1
     // loads of the step at q; CL: planes clamped to the grid
     auto load = [&](In& in, int q, auto clamp) {
       constexpr bool CL = decltype(clamp)::value;
@@ -139,40 +169,108 @@ __global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
         if constexpr (CL) return x[plane * sxy + (long long)(o / (unsigned)sizeof(T))];
         return *reinterpret_cast<const T*>(reinterpret_cast<const char*>(x + plane * sxy) + o);
       };
+      auto getk = [&](int a, int d, unsigned o) -> T {
+        const long long plane = CL ? min(max(q + a + d, 0), nz - 1) - a : q + d;
+        if constexpr (CL) return pair_k<T>(kf[plane * sxy + (long long)(o / (unsigned)sizeof(T))]);
+        return pair_k<T>(*reinterpret_cast<const KT*>(reinterpret_cast<const char*>(kf + plane * sxy) +
+                                                      o / (unsigned)(sizeof(T) / sizeof(KT))));
+      };
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const int a = (r & 1) ? 1 - a0 : a0;
+        if constexpr (kK) {
+          in.kc[r] = getk(a, 0, ro[r]);
+          in.kp[r] = getk(a, 1, ro[r]);
+          in.ke[r] = edge ? getk(a, 0, ro[r] + eo) : T(0);
+        }
         in.zp[r] = ZERO ? T(0) : get(xin, a, 1, ro[r]);
         in.xe[r] = !ZERO && edge ? get(xin, a, 0, ro[r] + eo) : T(0);
         in.b1[r] = get(b, a, 0, ro[r]);
         in.b2[r] = get(b, a, -1, ro[r]);
       }
       in.ylo = ZERO ? T(0) : get(xin, a0, 0, lo);
-      in.yhi = ZERO ? T(0) : get(xin, ((R - 1) & 1) ? 1 - a0 : a0, 0, hi);
+      const int ah = ((R - 1) & 1) ? 1 - a0 : a0;
+      in.yhi = ZERO ? T(0) : get(xin, ah, 0, hi);
+      if constexpr (kK) {
+        in.kl[0] = getk(a0, 0, lo);
+        in.kl[1] = getk(a0, -1, lo);
+        in.kh[0] = getk(ah, 0, hi);
+        in.kh[1] = getk(ah, -1, hi);
+      }
     };
-    const Stencil<T> st = cf.template at<T, 3>(GridDev{}, 0);
-    PairDiv<T> dv[R];  // by the centre of each row with its x and y closures
-    T least = PairDiv<T>::kLeast;
+    Stencil<T> st;
+    if constexpr (!kK) st = cf.template at<T, 3>(GridDev{}, 0);
+    PairDiv<T> dv[kK ? 1 : R];  // by the centre of each row with its x and y closures
+    T least[kK ? 1 : R];  // range test of the dividends: below any value on other rows (their zeros are not divided)
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int a = (r & 1) ? 1 - a0 : a0;
-      zm[r] = ZERO ? T(0)
-                   : xin[(long long)(min(max(p + a - 1, 0), nz - 1) - a) * sxy +
-                         (long long)(ro[r] / (unsigned)sizeof(T))];
+      auto pl = [&](int d) {
+        return (long long)(min(max(p + a + d, 0), nz - 1) - a) * sxy + (long long)(ro[r] / (unsigned)sizeof(T));
+      };
+      zm[r] = ZERO ? T(0) : xin[pl(-1)];
       vp[r] = T(0);
-      T c = st.c;
-      c += st.xm * fxl;
-      c += st.xp * fxh;
-      if (j0 + r == 1) c += st.ym * fyl;
-      if (j0 + r == ny - 2) c += st.yp * fyh;
-      dv[r].init(c, least);
-      if (!(inm >> r & 1)) dv[r].y = T(0);
+      if constexpr (kK) {
+        km[r] = pair_k<T>(kf[pl(-2)]);
+        kb[r] = pair_k<T>(kf[pl(-1)]);
+      } else {
+        T c = st.c;
+        c += st.xm * fxl;
+        c += st.xp * fxh;
+        if (j0 + r == 1) c += st.ym * fyl;
+        if (j0 + r == ny - 2) c += st.yp * fyh;
+        least[r] = PairDiv<T>::kLeast;
+        dv[r].init(c, least[r]);
+        if (!(inm >> r & 1)) {
+          dv[r].y = T(0);
+          least[r] = T(-1);
+        }
+      }
     }
+    // Value of the node of row r on plane P with k around it (CoefDivk::at with
+    // its factors 1/2 gathered, fold_faces, the general division). Other rows
+    // divide their centre by itself: a zero dividend takes the slow division.
+    auto from_k = [&](int r, bool zed, int P, T kc, T kxm, T kxp, T kym, T kyp, T kzm, T kzp, T bv, T xp, T xm, T yp, T ym,
+                      T zpv, T zmv) -> T {
+      if constexpr (kK) {
+        const T hx = T(0.5) * T(cf.ihx2), hy = T(0.5) * T(cf.ihy2), hz = T(0.5) * T(cf.ihz2);
+        const T sxm = kc + kxm, sxp = kc + kxp, sym = kc + kym, syp = kc + kyp, szm = kc + kzm, szp = kc + kzp;
+        Stencil<T> t;
+        t.xm = -sxm * hx - T(cf.cx);
+        t.xp = -sxp * hx + T(cf.cx);
+        t.ym = -sym * hy - T(cf.dyc);
+        t.yp = -syp * hy + T(cf.dyc);
+        t.zm = -szm * hz - T(cf.dzc);
+        t.zp = -szp * hz + T(cf.dzc);
+        T c = (sxm + sxp) * hx + (sym + syp) * hy;
+        c += (szm + szp) * hz;
+        c += T(cf.e);
+        c += t.xm * fxl;
+        c += t.xp * fxh;
+        if (j0 + r == 1) c += t.ym * fyl;
+        if (j0 + r == ny - 2) c += t.yp * fyh;
+        bool in = inm >> r & 1;
+        if (zed) {
+          if (P == 1) c += t.zm * fzl;
+          if (P == nz - 2) c += t.zp * fzh;
+          in = in && P >= 1 && P <= nz - 2;
+        }
+        const T n = bv - nb_sum<T>(t, xp, xm, yp, ym, zpv, zmv, 3);
+        T d = in ? n : c;
+        if constexpr (sizeof(T) == 8)
+          asm("" : "+d"(d));  // (the selections would be merged into one after the division)
+        else
+          asm("" : "+f"(d));
+        const T v = d / c;
+        return in ? v : T(0);
+      }
+      return T(0);
+    };
     // numerators to values, with one range test for all rows
     auto quotients = [&](T (&v)[R]) {
       bool ok = true;
 #pragma unroll
-      for (int r = 0; r < R; ++r) ok = ok && fabs(v[r]) >= least && fabs(v[r]) < PairDiv<T>::kMost;
+      for (int r = 0; r < R; ++r) ok = ok && fabs(v[r]) >= least[r] && fabs(v[r]) < PairDiv<T>::kMost;
       if (ok) {
 #pragma unroll
         for (int r = 0; r < R; ++r) v[r] = dv[r](v[r]);
@@ -209,9 +307,17 @@ __global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
           if constexpr (DOT) acc[0] += double(rhs) * double(val);
         }
       };
-      T s[R], v[R], w[R];
+      T s[R], v[R], w[R], s1[RK], s2[RK];  // (s1, s2: k on the neighbours' planes P and P - 1)
 #pragma unroll
       for (int r = 0; r < R; ++r) s[r] = ((r & 1) ? !a0 : a0) ? zm[r] : in.zp[r];  // as the neighbours read it
+      if constexpr (kK) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const bool a = (r & 1) ? !a0 : a0;
+          s1[r] = a ? kb[r] : in.kp[r];
+          s2[r] = a ? km[r] : in.kc[r];
+        }
+      }
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         T xl = T(0), xr = T(0), yl = T(0), yh = T(0);
@@ -223,9 +329,19 @@ __global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
           yl = r > 0 ? s[r > 0 ? r - 1 : 0] : in.ylo;
           yh = r < R - 1 ? s[r < R - 1 ? r + 1 : 0] : in.yhi;
         }
-        v[r] = in.b1[r] - nb_sum<T>(st, xr, xl, yh, yl, in.zp[r], zm[r], 3);
+        if constexpr (kK) {
+          T kl = __shfl_up_sync(kAll, s1[r], 1), kr = __shfl_down_sync(kAll, s1[r], 1);
+          if (lane == 0) kl = in.ke[r];
+          if (lane == 31) kr = in.ke[r];
+          v[r] = from_k(r, !HOT, (r & 1) ? po : pe, in.kc[r], kl, kr, r > 0 ? s1[r > 0 ? r - 1 : 0] : in.kl[0],
+                        r < R - 1 ? s1[r < R - 1 ? r + 1 : 0] : in.kh[0], kb[r], in.kp[r], in.b1[r], xr, xl, yh, yl,
+                        in.zp[r], zm[r]);
+        } else {
+          v[r] = in.b1[r] - nb_sum<T>(st, xr, xl, yh, yl, in.zp[r], zm[r], 3);
+        }
       }
-      if constexpr (HOT)
+      if constexpr (kK) {
+      } else if constexpr (HOT)
         quotients(v);
       else
         edge_quotients(v, pe, po);
@@ -242,9 +358,17 @@ __global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
       for (int r = 0; r < R; ++r) {
         const T xl = __shfl_up_sync(kAll, s[r], 1), xr = __shfl_down_sync(kAll, s[r], 1);
         const T yl = r > 0 ? s[r > 0 ? r - 1 : 0] : nlo, yh = r < R - 1 ? s[r < R - 1 ? r + 1 : 0] : nhi;
-        w[r] = in.b2[r] - nb_sum<T>(st, xr, xl, yh, yl, v[r], vp[r], 3);
+        if constexpr (kK) {
+          const T kl = __shfl_up_sync(kAll, s2[r], 1), kr = __shfl_down_sync(kAll, s2[r], 1);
+          w[r] = from_k(r, !HOT, ((r & 1) ? po : pe) - 1, kb[r], kl, kr, r > 0 ? s2[r > 0 ? r - 1 : 0] : in.kl[1],
+                        r < R - 1 ? s2[r < R - 1 ? r + 1 : 0] : in.kh[1], km[r], in.kc[r], in.b2[r], xr, xl, yh, yl, v[r],
+                        vp[r]);
+        } else {
+          w[r] = in.b2[r] - nb_sum<T>(st, xr, xl, yh, yl, v[r], vp[r], 3);
+        }
       }
-      if constexpr (HOT)
+      if constexpr (kK) {
+      } else if constexpr (HOT)
         quotients(w);
       else
         edge_quotients(w, pe - 1, po - 1);
@@ -253,6 +377,10 @@ __global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
         put(-1, r, w[r], in.b2[r]);
         zm[r] = in.zp[r];
         vp[r] = v[r];
+        if constexpr (kK) {
+          km[r] = in.kc[r];
+          kb[r] = in.kp[r];
+        }
       }
       buf ^= 1;
       p += 2;

@@ -569,13 +569,15 @@ struct Hierarchy {
   // 226 us per sweep on a box where a colour pass takes 113 us, so the colour
   // passes stay the default.
   static constexpr long long kMarchMinNodes = 1LL << 18;
-  // 3D levels of at least this many nodes with constant coefficients and closure
-  // factors per face smooth with k_rbgs_pair (PDEB200_PAIR_MIN sets the number):
-  // below, two colour passes out of L2 are faster. Convection-diffusion solves,
-  // with it against without: FP32 513^3 70 / 84 ms, 300^3 21.5 / 23.6, 257^3 13.8 /
-  // 14.4, 225^3 11.2 / 10.7; FP64 300^3 24.7 / 26.4, 257^3 16.9 / 17.3, 225^3 12.8 /
-  // 12.8, 171^3 7.8 / 7.1. A plane's byte offsets take 32 bits (sxy < 2^27).
-  static constexpr long long kPairMinNodes = 1LL << 24;
+  // 3D levels of at least this many nodes with constant or divergence-form
+  // coefficients and closure factors per face smooth with k_rbgs_pair
+  // (PDEB200_PAIR_MIN sets the number): below, two colour passes out of L2 are as
+  // fast or faster. Solves in ms, with it against without: divergence form FP64
+  // 257^3 16.9 / 18.9, 171^3 7.0 / 8.0, 129^3 4.02 / 3.99; BF16 k 257^3 15.8 / 16.8,
+  // 171^3 6.4 / 6.8, 129^3 3.93 / 3.91; convection-diffusion FP64 225^3 10.2 / 12.2,
+  // 171^3 6.3 / 6.6, 129^3 3.9 / 3.7; FP32 513^3 60 / 79, 171^3 6.2 / 6.7, 145^3 4.40 /
+  // 4.35. A plane's byte offsets take 32 bits (sxy < 2^27).
+  static constexpr long long kPairMinNodes = 3LL << 20;
   static constexpr bool kSweepCoef =
       std::is_same<T, double>::value &&
       (std::is_same<Coef, CoefConst>::value || std::is_same<Coef, CoefDivk<double>>::value);
@@ -803,7 +805,7 @@ struct Hierarchy {
                       L.g.n >= kSweepMinNodes;
       L.march = kSweepCoef && march_env && !fused && !L.single_pass && l + 1 < levels.size() && L.g.dim == 3 &&
                 L.g.n >= kMarchMinNodes;
-      L.pair = std::is_same<Coef, CoefConst>::value && !fused && !L.single_pass && !L.march && l + 1 < levels.size() &&
+      L.pair = PairK<Coef>::kOk && !fused && !L.single_pass && !L.march && l + 1 < levels.size() &&
                (int)l != cv_l0 && (int)l != tail_l0 && L.g.dim == 3 && L.g.n >= pair_min && L.g.sxy < (1LL << 27) &&
                ext_coef(L.g, &pair_ext);
       if (L.pair) {
@@ -836,10 +838,10 @@ struct Hierarchy {
     const dim3 grid = rbgs_grid(L.g), block = stencil_block();
     const dim3 zgrid = stencil_grid_auto(L.g);  // the pass from zero (fewer registers) keeps the default
     const double dofs = interior_dofs(L.g);
-    if constexpr (std::is_same<Coef, CoefConst>::value) {
+    if constexpr (PairK<Coef>::kOk) {
       if (L.pair) {
-        const dim3 pgrid = pair_grid(L.g, PairShape<T>::kRows, PairShape<T>::kMinBlocks);
-        const dim3 pblock(32 * PairShape<T>::W);
+        const dim3 pgrid = pair_grid(L.g, PairShape<Coef, T>::kRows, PairShape<Coef, T>::kMinBlocks);
+        const dim3 pblock(32 * PairShape<Coef, T>::W);
         const LevelGeo pg = level_geo(L.g);
         const PairFold pf = pair_fold(L.g);
         // from zero: the last sweep ends in xa
@@ -851,13 +853,13 @@ struct Hierarchy {
           ProfScope ps(ctx, zero ? "pair_sweep_zero" : "pair_sweep", lvl,
                        dofs * (zero ? 2.0 : 3.0) * sizeof(T));
           if (zero)
-            launch_dep(ctx, pgrid, pblock, 0, k_rbgs_pair<T, true, false, NoPost>, pg, pf, L.cf, b, in, out, first,
+            launch_dep(ctx, pgrid, pblock, 0, k_rbgs_pair<Coef, T, true, false, NoPost>, pg, pf, L.cf, b, in, out, first,
                        ctl, RedSlot{}, NoPost{});
           else if (dot_last && s + 1 == sweeps)
-            launch_dep(ctx, pgrid, pblock, 0, k_rbgs_pair<T, false, true, PostBeta>, pg, pf, L.cf, b, in, out, first,
+            launch_dep(ctx, pgrid, pblock, 0, k_rbgs_pair<Coef, T, false, true, PostBeta>, pg, pf, L.cf, b, in, out, first,
                        ctl, *dot_last, PostBeta{const_cast<Ctl*>(ctl)});
           else
-            launch_dep(ctx, pgrid, pblock, 0, k_rbgs_pair<T, false, false, NoPost>, pg, pf, L.cf, b, in, out, first,
+            launch_dep(ctx, pgrid, pblock, 0, k_rbgs_pair<Coef, T, false, false, NoPost>, pg, pf, L.cf, b, in, out, first,
                        ctl, RedSlot{}, NoPost{});
           ctx->count();
           cur = out;

@@ -91,3 +91,32 @@ def test_bicgstab_in_mixed_precision_on_column_kernels(monkeypatch, dims):
     a, b, ra, rb = both(monkeypatch, p, opt)
     assert ra.status == abi.OK and ra.rel_residual <= 1e-10
     assert np.linalg.norm(a - b) <= 1e-8 * np.linalg.norm(b)  # the bar of the mixed form
+
+
+def make_divk(dims):
+    p = make(dims)
+    q = GridProblem(*dims, coef_kind=abi.COEF_DIVK)
+    q.k = np.exp(0.5 * np.random.Generator(np.random.PCG64(7)).standard_normal(q.n))
+    q.f, q.faces = p.f, p.faces
+    return q
+
+
+@pytest.mark.parametrize("dims", DIMS)
+@pytest.mark.parametrize("sweeps", [(2, 2), (1, 2), (3, 1)])
+def test_one_pass_with_sampled_k(monkeypatch, dims, sweeps):
+    opt = default_options(method=abi.MG_PCG, tol=0.0, tol_mode=abi.TOL_RELATIVE, max_iter=2, mg_pre_smooth=sweeps[0],
+                          mg_post_smooth=sweeps[1])
+    a, b, ra, rb = both(monkeypatch, make_divk(dims), opt)
+    assert ra.iterations == rb.iterations
+    assert np.linalg.norm(a - b) <= 1e-11 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("dims", DIMS[:5])
+@pytest.mark.parametrize("bf16", [0, 1])
+def test_one_pass_with_sampled_k_in_mixed_precision(monkeypatch, dims, bf16):
+    opt = default_options(method=abi.MG_PCG, tol=1e-11, tol_mode=abi.TOL_RELATIVE, max_iter=200, precision=abi.MIXED,
+                          bf16_coefficients=bf16)
+    a, b, ra, rb = both(monkeypatch, make_divk(dims), opt)
+    assert ra.status == abi.OK and ra.rel_residual <= 1e-11
+    assert abs(ra.iterations - rb.iterations) <= 1
+    assert np.linalg.norm(a - b) <= 1e-8 * np.linalg.norm(b)
