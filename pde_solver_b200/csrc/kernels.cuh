@@ -935,14 +935,6 @@ __device__ __forceinline__ double ext_value(const GridDev& gc, const TC* __restr
   return coef == 0.0 ? 0.0 : coef * double(xc[cidx(gc, I, J, K)]);
 }
 
-// z-marching restriction for level pairs whose z map is the identity or
-// nested 2:1 (every odd side, and every 2D grid). One thread per column sums
-// each fine plane's x-y weights once and shares the plane sum between the two
-// coarse planes it feeds.
-__device__ __forceinline__ bool z_marchable(const GridDev& gf, const GridDev& gc) {
-  return gf.dim != 3 || map_mode(gf.nz, gc.nz) <= 1;
-}
-
 // Full weighting of one coarse column (I, J): the x-y weights once, then the
 // weighted sum of any fine plane.
 template <typename T>

@@ -56,11 +56,13 @@ using PairShape =
 template <class Coef>
 struct PairK {
   static constexpr bool kHas = false, kOk = std::is_same<Coef, CoefConst>::value;
+  static constexpr double kBytes = 0.0;
   __device__ static const float* field(const Coef&) { return nullptr; }
 };
 template <typename KT>
 struct PairK<CoefDivk<KT>> {
   static constexpr bool kHas = true, kOk = true;
+  static constexpr double kBytes = sizeof(KT);
   __device__ static const KT* field(const CoefDivk<KT>& c) { return c.k; }
 };
 template <typename T, typename KT>

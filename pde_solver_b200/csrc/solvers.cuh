@@ -427,8 +427,8 @@ inline bool coarse_dims(const GridDev& g, const pdeb200_problem* hp, int nc[3]) 
   return any;
 }
 
-// the z map of a level pair is the identity or nested 2:1 (host-side test of
-// z_marchable in kernels.cuh)
+// the z map of a level pair is the identity or nested 2:1: each fine plane's x-y
+// sum is shared by the two coarse planes it feeds
 inline bool z_nested(const GridDev& gf, const GridDev& gc) {
   return gf.dim != 3 || gc.nz == gf.nz || 2 * gc.nz - 1 == gf.nz;
 }
@@ -538,8 +538,9 @@ inline CoefNodal coarsen_coef(Context* ctx, const DevProblem&, const CoefNodal& 
 // (odd cubes nest 2:1 as in the reference's multigrid.cpp:150-170, continued
 // down to 3 nodes; even sizes use the non-nested maps of kernels.cuh); face
 // closures are rediscretised with the coarse spacing.
-// Each level has two field buffers: smoothing sweeps are fused red-black
-// passes that read one buffer and write the other.
+// Smoothing sweeps are colour passes in place, on large 3D levels one pass
+// between the field and the residual buffer (k_rbgs_pair); the option forms
+// have a second field buffer.
 template <class Coef, typename T>
 struct Hierarchy {
   struct Level {
@@ -829,9 +830,9 @@ struct Hierarchy {
   }
 
   // `sweeps` red-black sweeps starting from `cur` (or from zero); returns the
-  // buffer holding the result. Two forms with identical arithmetic: colour
-  // passes in place (default), or fused single-pass sweeps that read one
-  // buffer and write the other.
+  // buffer holding the result. Forms with identical arithmetic: colour passes
+  // in place, or single-pass sweeps that read one buffer and write the other
+  // (k_rbgs_pair by default on large levels, the others by option).
   bool fused = false;
   T* sweeps_from(Context* ctx, Level& L, const T* b, T* cur, int sweeps, int first, bool from_zero,
                  const Ctl* ctl, int lvl, const RedSlot* dot_last = nullptr) {
@@ -851,7 +852,7 @@ struct Hierarchy {
           T* out = cur == L.xa ? L.r : L.xa;
           const T* in = cur;
           ProfScope ps(ctx, zero ? "pair_sweep_zero" : "pair_sweep", lvl,
-                       dofs * (zero ? 2.0 : 3.0) * sizeof(T));
+                       dofs * ((zero ? 2.0 : 3.0) * sizeof(T) + PairK<Coef>::kBytes));
           if (zero)
             launch_dep(ctx, pgrid, pblock, 0, k_rbgs_pair<Coef, T, true, false, NoPost>, pg, pf, L.cf, b, in, out, first,
                        ctl, RedSlot{}, NoPost{});
