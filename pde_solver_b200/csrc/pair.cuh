@@ -25,10 +25,10 @@
 // Issue bound (about 110 instructions per lane and column step, 63% of the
 // issue slots), then DRAM: FP32 513^3 421 us per sweep against 737 for two colour
 // passes (250 at the copy rate); FP64 257^3 101 against 162, 300^3 139 against 261.
-// Divergence form: k of the neighbours by shuffles too; FP64 257^3 177 us against
-// 226, BF16 k in FP32 125 against 141. Lanes off the interior keep ordinary
+// Divergence form: k of the neighbours by shuffles too; FP64 257^3 169 us against
+// 226, BF16 k in FP32 126 against 145. Lanes off the interior keep ordinary
 // dividends: zeros take the division's slow branch and held whole blocks up (258
-// instead of 177).
+// instead of 177 in the 3 x 8 x 1 shape).
 #pragma once
 
 #include "cluster.cuh"
@@ -40,17 +40,20 @@ constexpr int kPairCols = 30;  // columns a warp writes
 // Rows per lane, warps per block and blocks per SM. FP32 at 513^3: 4 x 8 x 2
 // 421 us, 4 x 4 x 5 418 (spills), 3 x 8 x 3 443, 6 x 4 x 3 425, 8 x 4 x 3 501;
 // FP64 at 257^3 / 300^3: 3 x 8 x 2 101 / 139, 2 x 16 x 1 111 / 153, 2 x 8 x 2
-// 107 / 152, 3 x 4 x 4 101 / 154. Divergence form FP64 at 257^3: 3 x 8 x 1 177, 2 x 8 x
-// 2 209 (spills), 4 x 4 x 2 183, 3 x 4 x 3 205, 4 x 8 x 1 195.
+// 107 / 152, 3 x 4 x 4 101 / 154. Divergence form at 257^3, a sweep / one from
+// zero: FP64 2 x 12 x 1 169 / 135, 3 x 8 x 1 178 / 152, 2 x 8 x 2 209 (spills), 4 x 4
+// x 2 183, 3 x 10 x 1 271 (spills); BF16 k 3 x 8 x 2 126 / 105, 4 x 8 x 2 131 / 113,
+// 4 x 4 x 3 128 / 98, 2 x 8 x 3 130 / 105, 4 x 8 x 1 156 / 140.
 template <int R_, int W_, int B_>
 struct PairShapeOf {
   static constexpr int R = R_, W = W_, kMinBlocks = B_;
   static constexpr int kRows = R_ * W_ - 2;  // rows a block writes
 };
 template <class Coef, typename T>
-using PairShape =
-    std::conditional_t<sizeof(T) == 4, PairShapeOf<4, 8, 2>,
-                       std::conditional_t<std::is_same<Coef, CoefConst>::value, PairShapeOf<3, 8, 2>, PairShapeOf<3, 8, 1>>>;
+using PairShape = std::conditional_t<
+    std::is_same<Coef, CoefConst>::value,
+    std::conditional_t<sizeof(T) == 4, PairShapeOf<4, 8, 2>, PairShapeOf<3, 8, 2>>,
+    std::conditional_t<sizeof(T) == 4, PairShapeOf<3, 8, 2>, PairShapeOf<2, 12, 1>>>;
 
 // k of divergence-form coefficients
 template <class Coef>
@@ -229,11 +232,12 @@ __global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
         }
       }
     }
-    // Value of the node of row r on plane P with k around it (CoefDivk::at with
+    // Value of the node of row r on plane P with k around it (zero: of a zero field;
+    // CoefDivk::at with
     // its factors 1/2 gathered, fold_faces, the general division). Other rows
     // divide their centre by itself: a zero dividend takes the slow division.
     auto from_k = [&](int r, bool zed, int P, T kc, T kxm, T kxp, T kym, T kyp, T kzm, T kzp, T bv, T xp, T xm, T yp, T ym,
-                      T zpv, T zmv) -> T {
+                      T zpv, T zmv, auto zero) -> T {
       if constexpr (kK) {
         const T hx = T(0.5) * T(cf.ihx2), hy = T(0.5) * T(cf.ihy2), hz = T(0.5) * T(cf.ihz2);
         const T sxm = kc + kxm, sxp = kc + kxp, sym = kc + kym, syp = kc + kyp, szm = kc + kzm, szp = kc + kzp;
@@ -257,7 +261,8 @@ __global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
           if (P == nz - 2) c += t.zp * fzh;
           in = in && P >= 1 && P <= nz - 2;
         }
-        const T n = bv - nb_sum<T>(t, xp, xm, yp, ym, zpv, zmv, 3);
+        T n = bv;
+        if constexpr (!decltype(zero)::value) n = bv - nb_sum<T>(t, xp, xm, yp, ym, zpv, zmv, 3);
         T d = in ? n : c;
         if constexpr (sizeof(T) == 8)
           asm("" : "+d"(d));  // (the selections would be merged into one after the division)
@@ -337,9 +342,10 @@ __global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
           if (lane == 31) kr = in.ke[r];
           v[r] = from_k(r, !HOT, (r & 1) ? po : pe, in.kc[r], kl, kr, r > 0 ? s1[r > 0 ? r - 1 : 0] : in.kl[0],
                         r < R - 1 ? s1[r < R - 1 ? r + 1 : 0] : in.kh[0], kb[r], in.kp[r], in.b1[r], xr, xl, yh, yl,
-                        in.zp[r], zm[r]);
+                        in.zp[r], zm[r], std::integral_constant<bool, ZERO>{});
         } else {
-          v[r] = in.b1[r] - nb_sum<T>(st, xr, xl, yh, yl, in.zp[r], zm[r], 3);
+          v[r] = in.b1[r];
+          if constexpr (!ZERO) v[r] = in.b1[r] - nb_sum<T>(st, xr, xl, yh, yl, in.zp[r], zm[r], 3);
         }
       }
       if constexpr (kK) {
@@ -364,7 +370,7 @@ __global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
           const T kl = __shfl_up_sync(kAll, s2[r], 1), kr = __shfl_down_sync(kAll, s2[r], 1);
           w[r] = from_k(r, !HOT, ((r & 1) ? po : pe) - 1, kb[r], kl, kr, r > 0 ? s2[r > 0 ? r - 1 : 0] : in.kl[1],
                         r < R - 1 ? s2[r < R - 1 ? r + 1 : 0] : in.kh[1], km[r], in.kc[r], in.b2[r], xr, xl, yh, yl, v[r],
-                        vp[r]);
+                        vp[r], std::false_type{});
         } else {
           w[r] = in.b2[r] - nb_sum<T>(st, xr, xl, yh, yl, v[r], vp[r], 3);
         }

@@ -574,9 +574,9 @@ struct Hierarchy {
   // coefficients and closure factors per face smooth with k_rbgs_pair
   // (PDEB200_PAIR_MIN sets the number): below, two colour passes out of L2 are as
   // fast or faster. Solves in ms, with it against without: divergence form FP64
-  // 257^3 16.9 / 18.9, 171^3 7.0 / 8.0, 129^3 4.02 / 3.99; BF16 k 257^3 15.8 / 16.8,
+  // 257^3 16.6 / 18.9, 171^3 6.9 / 8.0, 129^3 4.02 / 3.99; BF16 k 257^3 15.7 / 16.8,
   // 171^3 6.4 / 6.8, 129^3 3.93 / 3.91; convection-diffusion FP64 225^3 10.2 / 12.2,
-  // 171^3 6.3 / 6.6, 129^3 3.9 / 3.7; FP32 513^3 60 / 79, 171^3 6.2 / 6.7, 145^3 4.40 /
+  // 171^3 6.3 / 6.6, 129^3 3.9 / 3.7; FP32 513^3 59 / 79, 171^3 6.2 / 6.7, 145^3 4.40 /
   // 4.35. A plane's byte offsets take 32 bits (sxy < 2^27).
   static constexpr long long kPairMinNodes = 3LL << 20;
   static constexpr bool kSweepCoef =
