@@ -594,7 +594,7 @@ pdeb200_status gmres_reference(Context* ctx, DevProblem& P, const Coef& cf, cons
 template <class Coef, class HierT, typename T>
 struct MgBicgCore {
   Buf buf;
-  StepGraph graph;
+  StepGraph graph{true};  // its first search direction is r
 
   pdeb200_status run(Context* ctx, HierT& H, const GridDev& g, const Coef& cf, const T* b, T* x, int max_iter,
                      double tol, const pdeb200_options* o, int* iters) {
@@ -760,7 +760,7 @@ __global__ void k_add_scaled(long long n, double* __restrict__ x, const T* __res
 template <class Coef, class HierT, typename T>
 struct MgPcgCore {
   Buf buf;
-  StepGraph graph;
+  StepGraph graph{false};
 
   pdeb200_status run(Context* ctx, HierT& H, const GridDev& g, const Coef& cf, const T* b, T* x, int max_iter,
                      double tol, const pdeb200_options* o, int* iters) {

@@ -230,7 +230,7 @@ pdeb200_status mg_pcg(Context* ctx, DevProblem& P, const Coef& cf, const pdeb200
     }
     ctx->count(2);
   };
-  StepGraph graph;
+  StepGraph graph{false};
   auto step = [&](int it) { graph.step(ctx, n, it, iterate, iterate); };
   // |r|^2 <= tol2 on the device (PostRRRel): batches sized by the observed reduction rate
   pdeb200_status st = drive(ctx, o, max_iter + 1, step, false, true);

@@ -288,14 +288,18 @@ struct IterGraph {
 struct StepGraph {
   static constexpr long long kDirectLaunches = 24;
   static constexpr long long kDirectNodes = 1LL << 20;
+  // iteration 0 of every solve starts otherwise than the replayed one (an
+  // object that serves several solves launches each solve's first directly)
+  const bool first_differs;
   IterGraph graph;
   int state = -1;  // -1 not tried, 0 direct, 1 replay
   long long launches = 0;
+  explicit StepGraph(bool differs) : first_differs(differs) {}
   // `first`: enqueues iteration `it` directly; `repeat`: the one to replay
   template <class First, class Repeat>
   void step(Context* ctx, long long n, int it, First&& first, Repeat&& repeat) {
     if (state < 0 && it >= 2 && launches > kDirectLaunches && n <= kDirectNodes) state = graph.capture(ctx, repeat) ? 1 : 0;
-    if (state == 1) {
+    if (state == 1 && !(first_differs && it == 0)) {
       graph.launch(ctx);
       return;
     }

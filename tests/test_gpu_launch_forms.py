@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 
 from pde_solver_b200 import abi, solver, synthetic
-from pde_solver_b200.problem import FaceBC, default_options
+from pde_solver_b200.problem import FaceBC, GridProblem, default_options
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +65,21 @@ def test_programmatic_launch_changes_no_numbers(tmp_path):
     assert res.returncode == 0, res.stderr[-2000:]
     assert int(res.stdout.strip().splitlines()[-1]) == ra.iterations
     assert np.array_equal(np.load(out), a)
+
+
+# Several inner solves per refinement, each of three and more iterations: every
+# one starts from its own residual, whether its iterations are replayed or not.
+# Levels by launches, so that an iteration has enough of them to be captured.
+@pytest.mark.parametrize("dims", [(49, 49, 49), (41, 53, 37), (150, 140, 1)])
+def test_graph_replay_changes_no_numbers_in_refinement(monkeypatch, dims):
+    nx, ny, nz = dims
+    p = GridProblem(nx, ny, nz, a=-1.0, b=-1.0, az=-1.0, c=30.0, d=-20.0, dz=10.0 if nz > 1 else 0.0)
+    p.f = np.random.Generator(np.random.PCG64(nx)).standard_normal(p.n)
+    opt = default_options(method=abi.MG_BICGSTAB, precision=abi.MIXED, tol=1e-12, tol_mode=abi.TOL_RELATIVE,
+                          max_iter=400)
+    monkeypatch.setenv("PDEB200_NO_TAIL", "1")
+    a, ra = solver.solve(p, opt)
+    monkeypatch.setenv("PDEB200_NO_GRAPH", "1")
+    b, rb = solver.solve(p, opt)
+    assert ra.status == abi.OK and ra.iterations == rb.iterations and ra.iterations >= 6
+    assert np.array_equal(a, b)
