@@ -463,11 +463,14 @@ __global__ void __launch_bounds__(kClusterThreads + 32) k_cluster_sweep(GridDev 
             double u_t = ut_zero ? 0.0 : v[m];
             if (!isfinite(u_t)) u_t = 0.0;
             v[m] = old_u[m] + a.dt * u_t;
-          } else {
-            const double du = fabs(v[m] - old_u[m]);  // a repeated last node changes no maximum
-            if (du > acc) acc = du;
           }
           if (q0 + m * nt < cnt) {
+            // (not of a repeated last node: another thread sends its copy, so the
+            // neighbour may already be writing the next sweep's values around it)
+            if constexpr (!HEAT) {
+              const double du = fabs(v[m] - old_u[m]);
+              if (du > acc) acc = du;
+            }
             *reinterpret_cast<double*>(dst + (e[m] & kClOffMask)) = v[m];
             if (e[m] >> kClFaceShift) {
               const unsigned faces = (e[m] >> kClFaceShift) & 63u;

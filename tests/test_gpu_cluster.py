@@ -75,6 +75,21 @@ def test_cluster_relaxation_sweep_counts(oracle_mod, method, sweeps):
     check(oracle_mod, make((23, 18, 1)), method=method, max_iter=sweeps, tol=0.0)
 
 
+# The last maximum is the one of the field's own nodes, to the bit: the fields of
+# S and S - 1 sweeps give it. Slabs whose threads have one node fewer than
+# others, on several CTAs.
+@pytest.mark.parametrize("dims", [(36, 35, 1), (97, 65, 1), (131, 67, 1), (129, 129, 1), (20, 19, 35)])
+@pytest.mark.parametrize("sweeps", [2, 41, 150])
+def test_cluster_jacobi_last_delta_is_of_the_field(dims, sweeps):
+    p = make(dims)
+    a, ra = solver.solve(p, default_options(method=abi.JACOBI, max_iter=sweeps, tol=0.0))
+    b, rb = solver.solve(p, default_options(method=abi.JACOBI, max_iter=sweeps - 1, tol=0.0))
+    inner = (slice(1, -1),) * (3 if dims[2] > 1 else 2)
+    shape = (dims[2], dims[1], dims[0]) if dims[2] > 1 else (dims[1], dims[0])
+    assert ra.iterations == sweeps and rb.iterations == sweeps - 1
+    assert ra.last_delta == np.abs(a - b).reshape(shape)[inner].max()
+
+
 @pytest.mark.parametrize("method", [abi.JACOBI, abi.SOR])
 @pytest.mark.parametrize("tol", [1.0, 1e-2, 1e-3, 1e-5, 1e-7])
 @pytest.mark.parametrize("dims", [(31, 44, 1), (13, 14, 15)])
