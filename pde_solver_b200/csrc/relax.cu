@@ -419,6 +419,7 @@ __global__ void __launch_bounds__(kClusterThreads + 32) k_cluster_lex(GridDev g,
       const bool late = (cl_load_u32(cl_map(&flags, 0)) & 2u) != 0;
       cl_sync(csize);
       const int pass = (int)first_pass;
+      __syncthreads();  // read by all before the next batch sets it
       if (pass < M) {
         for (int t = tid; t < local; t += nt) x[t] = save[t];
         cl_sync(csize);

@@ -90,6 +90,23 @@ def test_cluster_jacobi_last_delta_is_of_the_field(dims, sweeps):
     assert ra.last_delta == np.abs(a - b).reshape(shape)[inner].max()
 
 
+# A batch shorter than the one before it (the last before the sweep limit: 64,
+# 128 .. 512 sweeps, then 1 or 2): every warp takes the same branch after each
+# batch. One launch form only, so each run gives the same bits; against the
+# oracle once.
+@pytest.mark.parametrize("dims", [(36, 35, 1), (97, 65, 1), (20, 19, 35)])
+@pytest.mark.parametrize("sweeps", [66, 67, 194, 450, 963])
+def test_cluster_lexicographic_short_last_batch(oracle_mod, dims, sweeps):
+    p = make(dims)
+    opt = default_options(method=abi.SOR, max_iter=sweeps, tol=0.0)
+    check(oracle_mod, p, method=abi.SOR, max_iter=sweeps, tol=0.0)
+    first, r0 = solver.solve(p, opt)
+    for _ in range(10):
+        got, rep = solver.solve(p, opt)
+        assert (rep.iterations, rep.last_delta) == (r0.iterations, r0.last_delta)
+        assert np.array_equal(got, first)
+
+
 @pytest.mark.parametrize("method", [abi.JACOBI, abi.SOR])
 @pytest.mark.parametrize("tol", [1.0, 1e-2, 1e-3, 1e-5, 1e-7])
 @pytest.mark.parametrize("dims", [(31, 44, 1), (13, 14, 15)])
