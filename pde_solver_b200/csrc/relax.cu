@@ -436,6 +436,9 @@ __global__ void __launch_bounds__(kClusterThreads + 32) k_cluster_lex(GridDev g,
     } else if (phase == kRerun) {
       done += M;
       phase = kLast;
+      // the last sweep may begin with the parity that this one ended with: the
+      // copies of both steps go to the same places, so the first have to be there
+      cl_sync(csize);
     } else {
       acc = warp_max_nonneg(acc);
       if (lane == 0 && !control) wmax[warp] = acc;

@@ -107,6 +107,21 @@ def test_cluster_lexicographic_short_last_batch(oracle_mod, dims, sweeps):
         assert np.array_equal(got, first)
 
 
+# Stopping inside a batch with one plane per CTA and an odd last hyperplane: the
+# sweeps that are run again and the last one send the same nodes in a row.
+@pytest.mark.parametrize("dims", [(21, 18, 18), (18, 21, 18), (22, 18, 18)])
+@pytest.mark.parametrize("tol", [1e-2, 1e-4, 1e-6])
+def test_cluster_lexicographic_rerun_then_last_sweep(oracle_mod, dims, tol):
+    p = make(dims)
+    opt = default_options(method=abi.SOR, max_iter=20000, tol=tol)
+    check(oracle_mod, p, method=abi.SOR, max_iter=20000, tol=tol)
+    first, r0 = solver.solve(p, opt)
+    for _ in range(10):
+        got, rep = solver.solve(p, opt)
+        assert (rep.iterations, rep.last_delta) == (r0.iterations, r0.last_delta)
+        assert np.array_equal(got, first)
+
+
 @pytest.mark.parametrize("method", [abi.JACOBI, abi.SOR])
 @pytest.mark.parametrize("tol", [1.0, 1e-2, 1e-3, 1e-5, 1e-7])
 @pytest.mark.parametrize("dims", [(31, 44, 1), (13, 14, 15)])
