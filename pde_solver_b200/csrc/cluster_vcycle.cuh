@@ -513,8 +513,12 @@ __device__ __forceinline__ bool cv_cycle(const unsigned char* __restrict__ image
         }
         __syncthreads();
       }
+      // The first colour is sent to the neighbours, for the second colour's pass,
+      // which sends the second colour itself: a copy of it now would go to the
+      // same places with nothing to order the two. Without a pass to come none is
+      // sent.
       if (control) {
-        if (h.dist) exchange(h.expect[0] + h.expect[1]);
+        if (h.dist && post > 0) exchange(h.expect[0]);
       } else {
         for (int t = tid; t < 2 * h.cnt; t += nu) {
           const unsigned e = h.tab[t];
@@ -570,12 +574,12 @@ __device__ __forceinline__ bool cv_cycle(const unsigned char* __restrict__ image
           }
           const T nv = T(double(h.x[off]) + v);
           h.x[off] = nv;
-          if (e & (kClPrev | kClNext)) push(e, nv);
+          if (post > 0 && t < h.cnt && (e & (kClPrev | kClNext))) push(e, nv);
         }
       }
       __syncthreads();
     }
-    if (h.dist) ++step;
+    if (h.dist && post > 0) ++step;
     for (int p = 0; p < post; ++p) {
       pass(1, false);
       pass(0, false);

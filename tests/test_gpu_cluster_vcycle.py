@@ -60,6 +60,22 @@ def test_cluster_levels_match_launches(monkeypatch, dims, coef, faces, sweeps):
     assert rel_l2(a, b) <= 1e-11
 
 
+# What a CTA sends after the prolongation (nothing without sweeps after it) and
+# in the sweeps that follow: one and two layers per CTA; every run gives the same bits.
+@pytest.mark.parametrize("dims", [(17, 17, 18), (33, 33, 33), (40, 36, 20), (33, 40, 1), (129, 97, 1)])
+@pytest.mark.parametrize("sweeps", [(2, 1), (1, 0), (1, 3)])
+def test_cluster_levels_after_prolongation(monkeypatch, dims, sweeps):
+    p = make(dims, "divk", MIXED)
+    opt = default_options(method=abi.MG_PCG, tol=0.0, tol_mode=abi.TOL_RELATIVE, max_iter=2, mg_pre_smooth=sweeps[0],
+                          mg_post_smooth=sweeps[1])
+    a, _ = solver.solve(p, opt, raise_on_error=False)
+    for _ in range(10):
+        assert np.array_equal(solver.solve(p, opt, raise_on_error=False)[0], a)
+    monkeypatch.setenv("PDEB200_NO_TAIL", "1")
+    b, _ = solver.solve(p, opt, raise_on_error=False)
+    assert rel_l2(a, b) <= 1e-11
+
+
 def test_cluster_levels_semi_coarsened(monkeypatch):
     p = make((65, 33, 9), "divk", MIXED, bounds=(0.0, 4.0, 0.0, 1.0, 0.0, 0.1))
     opt = default_options(method=abi.MG_PCG, tol=0.0, tol_mode=abi.TOL_RELATIVE, max_iter=2)
