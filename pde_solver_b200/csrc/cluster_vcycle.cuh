@@ -229,6 +229,7 @@ __device__ __forceinline__ bool cv_cycle(const unsigned char* __restrict__ image
                                          int ncoarse, const Go& go) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ unsigned long long mbs[2], mbi;
+  __shared__ unsigned image_lost;
   const unsigned csize = cl_size(), rank = cl_rank();
   constexpr int nu = NU;
   const int tid = threadIdx.x, lane = tid & 31;
@@ -256,7 +257,12 @@ __device__ __forceinline__ bool cv_cycle(const unsigned char* __restrict__ image
     *reinterpret_cast<uint4*>(smem + o) = make_uint4(0u, 0u, 0u, 0u);
   const double map0 = coarse_map[0];
   __syncthreads();
-  bool dead = !mb_wait(&mbi, 0u);  // later: a wait ran out (control warp)
+  // Without its image a CTA knows no sizes: it touches nothing, and after the
+  // first cluster barrier all CTAs leave.
+  const bool no_image = __syncthreads_or(!mb_wait(&mbi, 0u)) != 0;
+  if (no_image) mb_wait(&mbi, 0u);  // the copies may still be on their way
+  if (tid == 0) image_lost = no_image ? 1u : 0u;
+  bool dead = false;  // a wait ran out (control warp)
   const CvGeo* geo = reinterpret_cast<const CvGeo*>(smem);
   const CvMine* mine = reinterpret_cast<const CvMine*>(smem + sizeof(CvGeo) * nlev);
   auto X = [&](int l) { return reinterpret_cast<T*>(smem + geo[l].x); };
@@ -301,11 +307,12 @@ __device__ __forceinline__ bool cv_cycle(const unsigned char* __restrict__ image
   };
   // the values of slot t of a level
   auto slot = [&](const Here& h, int t) -> T* { return h.w + t + (t >> 5) * (32 * (kCvRows - 1)); };
-  Here h = enter(0);
+  Here h{};
+  if (!no_image) h = enter(0);
   grid_dep_wait();
   grid_dep_release();
   if (!go()) return false;  // the same in every CTA
-  {
+  if (!no_image) {
     const T* src = rhs0 + (long long)(h.lo - 1) * h.L;
     for (int t = tid; t < 2 * h.cnt; t += blockDim.x) {
       const unsigned e = h.tab[t];
@@ -313,6 +320,10 @@ __device__ __forceinline__ bool cv_cycle(const unsigned char* __restrict__ image
     }
   }
   cl_sync(csize);
+  if (__any_sync(0xffffffffu, lane < (int)csize && cl_load_u32(cl_map(&image_lost, lane)) != 0u)) {
+    cl_leave(csize);
+    return control && lane == 0 && no_image;
+  }
   int step = 0;  // exchanges so far (the same in every CTA)
   auto push = [&](unsigned e, T v) {
     const unsigned m = 8u * (unsigned)(step & 1), o = kT * (e & kClOffMask);
