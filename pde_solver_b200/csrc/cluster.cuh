@@ -177,7 +177,8 @@ __device__ __forceinline__ Slab make_slab(const GridDev& g, int c, int csize) {
 }
 
 // Cluster size and buffer sizes of a grid: the fewest CTAs that leave at most
-// `nodes_per_cta` interior nodes to each, up to 16 and one layer each, and
+// `nodes_per_cta` interior nodes to each, up to `most` (Context::max_cluster)
+// and one layer each, and
 // kClusterNodes nodes per thread. Measured at 129x129 (16 CTAs) per Jacobi
 // sweep: 2 nodes per thread 0.90 us, 4 nodes 1.08 us; at 97x65 per SOR solve
 // with 512 nodes per CTA 16.5 ms, with 1024 17.9 ms (a step visits half of
@@ -190,13 +191,13 @@ struct ClusterShape {
   int slots;      // cnt_max with every row padded to an even length
 };
 
-inline ClusterShape cluster_shape(const GridDev& g, int nodes_per_cta) {
+inline ClusterShape cluster_shape(const GridDev& g, int nodes_per_cta, int most) {
   const int layers = (g.dim == 3 ? g.nz : g.ny) - 2;
   const long long L = g.dim == 3 ? g.sxy : g.nx;
   const int rows = g.dim == 3 ? g.ny - 2 : 1;
   const long long WH = (long long)(g.nx - 2) * rows;
   ClusterShape c{1, 0, 0, 0, 0};
-  while (c.csize < kClusterMax && 2 * c.csize <= layers && WH * ((layers + c.csize - 1) / c.csize) > nodes_per_cta)
+  while (2 * c.csize <= most && 2 * c.csize <= layers && WH * ((layers + c.csize - 1) / c.csize) > nodes_per_cta)
     c.csize *= 2;
   const long long n = (layers + c.csize - 1) / c.csize;
   if ((n + 2) * L > kClusterSmem / 8) return ClusterShape{0, 0, 0, 0, 0};

@@ -30,18 +30,14 @@ struct ClusterBicgArgs {
   int iters, relative;
 };
 
-// false: the launches serve the grid
-inline bool bicg_fits(const GridDev& g) {
-  return g.dim == 2 && (g.n + 255) / 256 <= kBiBlocks &&
-         (long long)((g.nx + kBx - 1) / kBx) * ((g.ny + kBy - 1) / kBy) <= kBiBlocks;
-}
-
-// the fewest CTAs with one stencil block per virtual block, up to 16
-inline int bicg_csize(const GridDev& g) {
-  const int nS = ((g.nx + kBx - 1) / kBx) * ((g.ny + kBy - 1) / kBy);
+// The fewest CTAs with one stencil block per virtual block, up to `most`
+// (Context::max_cluster); 0: the launches serve the grid
+inline int bicg_csize(const GridDev& g, int most) {
+  const long long nS = (long long)((g.nx + kBx - 1) / kBx) * ((g.ny + kBy - 1) / kBy);
+  if (g.dim != 2 || (g.n + 255) / 256 > kBiBlocks || nS > kBiBlocks) return 0;
   int c = 1;
-  while (c < kClusterMax && 4 * c < nS) c *= 2;
-  return c;
+  while (2 * c <= most && 4 * c < nS) c *= 2;
+  return nS <= 4LL * c * kBiRounds ? c : 0;
 }
 
 constexpr size_t kBiSmem = sizeof(double) * 5 * kBiThreads * kBiRounds;

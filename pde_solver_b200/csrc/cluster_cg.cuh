@@ -47,12 +47,13 @@ struct CgShape {
   size_t smem;
 };
 
-inline CgShape cg_shape(int nx, int ny, int nz) {
+// most: Context::max_cluster
+inline CgShape cg_shape(int nx, int ny, int nz, int most) {
   const bool is3 = nz > 1;
   const int layers = is3 ? nz : ny;
   const long long L = is3 ? (long long)nx * ny : nx;
   CgShape c{1, 0, false, 0};
-  while (c.csize < kClusterMax && 2 * c.csize <= layers && L * ((layers + c.csize - 1) / c.csize) > 1024) c.csize *= 2;
+  while (2 * c.csize <= most && 2 * c.csize <= layers && L * ((layers + c.csize - 1) / c.csize) > 1024) c.csize *= 2;
   const long long m = (layers + c.csize - 1) / c.csize;
   // p with its halo layers, the neighbours' r layers, a flag byte per node
   const size_t base = sizeof(double) * (size_t)((m + 2) * L + 2 * L) + (size_t)(m * L + 7) / 8 * 8;

@@ -113,6 +113,10 @@ struct Context {
   size_t max_blocks = 0;
   int num_sms = 148;
   bool pdl = true;  // launch_dep launches carry programmatic stream serialization
+  // most CTAs of a cluster that can be resident with all of their SMs' shared
+  // memory (a power of two, at most kClusterMax): 16 need a GPC with that many
+  // free SMs, which a client limited to part of the GPU may not have
+  int max_cluster = 1;
   std::string name;
   std::mutex mu;
   long long launches = 0;

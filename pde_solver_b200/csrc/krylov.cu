@@ -286,12 +286,12 @@ pdeb200_status bicgstab_reference(Context* ctx, DevProblem& P, const Coef& cf, c
   k_dot<double, PostBiInit><<<nb, 256, 0, ctx->stream>>>(n, r, r, ctx->slot(), PostBiInit{C, relative}, nullptr);
   ctx->count();
   pdeb200_status st;
-  if (bicg_fits(g)) {
+  const int csize = bicg_csize(g, ctx->max_cluster);
+  if (csize > 0) {
     // the loop inside one cluster, the launches' bits: 97x81 nodal 12.3 -> 3.9 ms
     Buf more(sizeof(double) * (3 * n + 6 * kBiBlocks), ctx->stream);
     double* M = more.as<double>();
     const ClusterBicgArgs a{d_x, M, p, M + n, v, M + 2 * n, r, s, t, b, rhat, M + 3 * n, kBiIters, relative};
-    const int csize = bicg_csize(g);
     auto run = [&](int) {
       launch_cluster(ctx, csize, kBiThreads, kBiSmem, k_cluster_bicg<Coef>, g, cf, a, C);
       ctx->count();

@@ -147,7 +147,7 @@ pdeb200_status time_series_dev(Context* ctx, DevProblem& P, const pdeb200_time_o
   // grids whose slabs fit in the shared memory of a cluster (about 120k nodes
   // in 2D) run all steps between two frames in one launch: 257x257, 200 steps
   // with 5 frames 2.14 -> 0.93 ms
-  const ClusterShape cs = cluster_shape(g, 1024);
+  const ClusterShape cs = cluster_shape(g, 1024, ctx->max_cluster);
   const size_t smem = (2 * sizeof(double)) * (size_t)cs.buf_nodes +
                       (sizeof(unsigned) + sizeof(double)) * (size_t)cs.cnt_max;
   const bool clustered = cs.csize > 0 && smem <= kClusterDynSmem;
@@ -470,7 +470,7 @@ pdeb200_status project_dev(Context* ctx, int nx, int ny, int nz, double dx, doub
   ctx->count(8);
   pdeb200_options o{};
   pdeb200_status st;
-  const CgShape cs = cg_shape(nx, ny, g.nz);
+  const CgShape cs = cg_shape(nx, ny, g.nz, ctx->max_cluster);
   if (cs.csize > 0) {
     // the loop inside one cluster: 256x256 19.5 -> 4.9 us per iteration,
     // 500x450 81 -> 39 ms

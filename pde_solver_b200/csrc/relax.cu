@@ -514,7 +514,7 @@ pdeb200_status gauss_seidel(Context* ctx, DevProblem& P, const Coef& cf, const p
   if (o->gs_ordering == PDEB200_ORDER_REDBLACK)
     throw StatusFailure{PDEB200_ERR_UNSUPPORTED, "red-black ordering is offered through the MG forms"};
   const unsigned long long budget = 60ULL * 1000000000ULL;  // device-time guard of the single-launch forms: 60 s
-  const ClusterShape cs = cluster_shape(g, 512);
+  const ClusterShape cs = cluster_shape(g, 512, ctx->max_cluster);
   const size_t lex_smem = sizeof(double) * (size_t)cs.buf_nodes + (sizeof(double) + sizeof(uint2)) * (size_t)cs.slots;
   // grids whose slabs fit in the shared memory of a cluster (about 160k nodes
   // in 2D): 97x65 SOR 483 -> 16.5 ms, and no grid is faster in the one-block form

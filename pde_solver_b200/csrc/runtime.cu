@@ -37,6 +37,37 @@ Context* get_context(int dev) {
   return g_ctx[dev].get();
 }
 
+// Stands for the cluster kernels where the residency of their clusters is asked for.
+__global__ void __launch_bounds__(1024) k_cluster_probe() {}
+
+static int max_cluster_of_device() {
+  const char* env = std::getenv("PDEB200_MAX_CLUSTER");
+  const int limit = env && std::atoi(env) > 0 ? std::atoi(env) : kClusterMax;
+  PDEB_CUDA(cudaFuncSetAttribute(k_cluster_probe, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmem));
+  PDEB_CUDA(cudaFuncSetAttribute(k_cluster_probe, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  for (int csize = kClusterMax; csize > 1; csize /= 2) {
+    if (csize > limit) continue;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(csize);
+    cfg.blockDim = dim3(1024);
+    cfg.dynamicSmemBytes = kClusterSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = csize;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, k_cluster_probe, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      clusters = 0;
+    }
+    if (clusters > 0) return csize;
+  }
+  return 1;
+}
+
 void init_context(Context* c, int dev) {
   PDEB_CUDA(cudaSetDevice(dev));
   c->dev = dev;
@@ -45,6 +76,7 @@ void init_context(Context* c, int dev) {
   c->name = prop.name;
   c->num_sms = prop.multiProcessorCount;
   c->pdl = std::getenv("PDEB200_NO_PDL") == nullptr;
+  c->max_cluster = max_cluster_of_device();
   PDEB_CUDA(cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking));
   c->stream = c->own_stream;
   PDEB_CUDA(cudaEventCreate(&c->ev0));

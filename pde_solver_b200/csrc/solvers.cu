@@ -31,7 +31,7 @@ pdeb200_status jacobi(Context* ctx, DevProblem& P, const Coef& cf, const pdeb200
   // grids whose slabs fit in the shared memory of a cluster (about 120k nodes
   // in 2D): whole runs of sweeps in one launch,
   // 129x129 0.90 against 7.5 us per sweep as launches
-  const ClusterShape cs = cluster_shape(g, 1024);
+  const ClusterShape cs = cluster_shape(g, 1024, ctx->max_cluster);
   const size_t smem = (2 * sizeof(double)) * (size_t)cs.buf_nodes +
                       (sizeof(unsigned) + sizeof(double)) * (size_t)cs.cnt_max;
   if (cs.csize > 0 && smem <= kClusterDynSmem) {
@@ -132,7 +132,7 @@ pdeb200_status cg_reference(Context* ctx, DevProblem& P, const Coef& cf, const p
   }
   ctx->count(relative ? 2 : 1);
   pdeb200_status st;
-  const CgShape cs = cg_shape(g.nx, g.ny, g.nz);
+  const CgShape cs = cg_shape(g.nx, g.ny, g.nz, ctx->max_cluster);
   if (cs.csize > 0) {
     // the loop inside one cluster: 129x129 (31 iterations) 0.76 -> 0.17 ms, 513x400 6.7 -> 2.8 ms
     const ClusterCgArgs a{d_x, r, p, q, kClusterCgIters, g.nx, g.ny, g.nz, relative ? 1 : 0, n};

@@ -680,7 +680,7 @@ struct Hierarchy {
       CvLayout lay;
       bool fits = false;
       for (int single : {512, 64}) {
-        csize = interior_dofs(levels[l].g) > single ? kClusterMax : 1;
+        csize = interior_dofs(levels[l].g) > single ? ctx->max_cluster : 1;
         lay = cv_layout<T>(gs.data(), n - l, csize, single, geo.data());
         fits = lay.total <= kCvSmem;
         if (fits) break;
