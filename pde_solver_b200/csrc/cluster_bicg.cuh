@@ -20,7 +20,7 @@ namespace pdeb {
 constexpr int kBiThreads = 1024;            // four virtual blocks
 constexpr int kBiBlocks = 256;              // most virtual blocks (the last tree is one block of 256 threads)
 constexpr int kBiRounds = kBiBlocks / (kClusterMax * 4);
-constexpr int kBiIters = 1024;              // iterations per launch; the host polls and sees a cancel between launches
+constexpr int kBiIters = 1024;              // most iterations per launch
 
 struct ClusterBicgArgs {
   double *x, *x1;                // field and its second buffer

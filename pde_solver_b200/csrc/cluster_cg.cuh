@@ -20,7 +20,7 @@
 
 namespace pdeb {
 
-constexpr int kClusterCgIters = 1024;  // iterations per launch; the host polls and sees a cancel between launches
+constexpr int kClusterCgIters = 1024;  // most iterations per launch
 
 constexpr int kCgThreads = 512;  // that update nodes; one more warp controls
 constexpr int kCgNodes = 4;       // nodes of a thread in flight at once

@@ -291,14 +291,13 @@ pdeb200_status bicgstab_reference(Context* ctx, DevProblem& P, const Coef& cf, c
     // the loop inside one cluster, the launches' bits: 97x81 nodal 12.3 -> 3.9 ms
     Buf more(sizeof(double) * (3 * n + 6 * kBiBlocks), ctx->stream);
     double* M = more.as<double>();
-    const ClusterBicgArgs a{d_x, M, p, M + n, v, M + 2 * n, r, s, t, b, rhat, M + 3 * n, kBiIters, relative};
-    auto run = [&](int) {
+    ClusterBicgArgs a{d_x, M, p, M + n, v, M + 2 * n, r, s, t, b, rhat, M + 3 * n, 0, relative};
+    auto run = [&](int iters) {
+      a.iters = iters;
       launch_cluster(ctx, csize, kBiThreads, kBiSmem, k_cluster_bicg<Coef>, g, cf, a, C);
       ctx->count();
     };
-    pdeb200_options po = *o;
-    po.check_interval = 1;
-    st = drive(ctx, &po, max_iter / kBiIters + 1, run, false);
+    st = drive_runs(ctx, o, max_iter, 1, kBiIters, run, false);
   } else {
     const dim3 grid = stencil_grid_full(g), block = stencil_block();
     auto iterate = [&](int it) {

@@ -23,6 +23,7 @@ pdeb200_status jacobi(Context* ctx, DevProblem& P, const Coef& cf, const pdeb200
                       pdeb200_report* rep) {
   const GridDev& g = P.g;
   const int max_iter = o->max_iter > 1 ? o->max_iter : 1;
+  constexpr int kJacobiGroup = 8;  // sweeps of a replayed graph, and between polls at first
   Buf degen(sizeof(int), ctx->stream);
   PDEB_CUDA(cudaMemsetAsync(degen.as<int>(), 0, sizeof(int), ctx->stream));
   PDEB_CUDA(cudaMemsetAsync(d_out, 0, sizeof(double) * g.n, ctx->stream));
@@ -35,18 +36,16 @@ pdeb200_status jacobi(Context* ctx, DevProblem& P, const Coef& cf, const pdeb200
   const size_t smem = (2 * sizeof(double)) * (size_t)cs.buf_nodes +
                       (sizeof(unsigned) + sizeof(double)) * (size_t)cs.cnt_max;
   if (cs.csize > 0 && smem <= kClusterDynSmem) {
-    constexpr int kSweepsPerLaunch = 2048;  // the host polls and sees a cancel between launches
+    constexpr int kSweepsPerLaunch = 2048;
     ClusterSweepArgs a{P.f, P.f_const, o->tol, max_iter, 0.0, 0.0, 0, cs.buf_nodes, cs.cnt_max};
     auto kern = g.dim == 3 ? (P.nl.n ? k_cluster_sweep<3, Coef, false, true> : k_cluster_sweep<3, Coef, false, false>)
                            : (P.nl.n ? k_cluster_sweep<2, Coef, false, true> : k_cluster_sweep<2, Coef, false, false>);
-    auto run = [&](int q) {
-      a.steps = std::min(kSweepsPerLaunch, max_iter - q * kSweepsPerLaunch);
+    auto run = [&](int sweeps) {
+      a.steps = sweeps;
       launch_cluster(ctx, cs.csize, cs.threads, smem, kern, g, cf, a, P.nl, d_out, ctx->d_ctl, degen.as<int>());
       ctx->count();
     };
-    pdeb200_options po = *o;
-    po.check_interval = 1;
-    const pdeb200_status st = drive(ctx, &po, (max_iter + kSweepsPerLaunch - 1) / kSweepsPerLaunch, run, true);
+    const pdeb200_status st = drive_runs(ctx, o, max_iter, kJacobiGroup, kSweepsPerLaunch, run, true);
     fill_boundary(ctx, g, d_out, nullptr);  // edges and corners
     const Ctl c = *ctx->h_ctl;
     int dg = 0;
@@ -76,7 +75,6 @@ pdeb200_status jacobi(Context* ctx, DevProblem& P, const Coef& cf, const pdeb200
   // captured once as a CUDA graph and replayed: small grids are launch-bound
   // (129^2: about 11 us per sweep as two direct launches). Sweeps after the
   // stopping test fired return at once, so a group may end past it.
-  constexpr int kJacobiGroup = 8;
   auto group = [&](int) {
     for (int t = 0; t < kJacobiGroup; ++t) iterate(t);
   };
@@ -135,15 +133,14 @@ pdeb200_status cg_reference(Context* ctx, DevProblem& P, const Coef& cf, const p
   const CgShape cs = cg_shape(g.nx, g.ny, g.nz, ctx->max_cluster);
   if (cs.csize > 0) {
     // the loop inside one cluster: 129x129 (31 iterations) 0.76 -> 0.17 ms, 513x400 6.7 -> 2.8 ms
-    const ClusterCgArgs a{d_x, r, p, q, kClusterCgIters, g.nx, g.ny, g.nz, relative ? 1 : 0, n};
+    ClusterCgArgs a{d_x, r, p, q, 0, g.nx, g.ny, g.nz, relative ? 1 : 0, n};
     auto kern = cluster_cg_kernel<kCgFull, Coef>(cs);
-    auto run = [&](int) {
+    auto run = [&](int iters) {
+      a.iters = iters;
       launch_cluster(ctx, cs.csize, cs.threads, cs.smem, kern, g, cf, CgProj{}, a, ctx->d_ctl);
       ctx->count();
     };
-    pdeb200_options po = *o;
-    po.check_interval = 1;
-    st = drive(ctx, &po, max_iter / kClusterCgIters + 1, run, false);
+    st = drive_runs(ctx, o, max_iter, 1, kClusterCgIters, run, false);
   } else {
     const dim3 grid = stencil_grid_full(g), block = stencil_block();
     auto iterate = [&](int) {

@@ -216,6 +216,33 @@ pdeb200_status drive(Context* ctx, const pdeb200_options* o, int max_iter, It&& 
   }
 }
 
+// drive() for kernels that make many iterations per launch: run(count) launches
+// the next `count` of `total`, at most `per_launch`. What the host looks for
+// between launches is a cancel, so they are short only with a cancel flag: they
+// then end where drive() polls after batches of `unit` iterations.
+template <class Run>
+pdeb200_status drive_runs(Context* ctx, const pdeb200_options* o, long long total, int unit, int per_launch, Run&& run,
+                          bool use_stop) {
+  const long long cap = o->check_interval > 0 ? o->check_interval : 16;
+  long long enq = 0, batch = 1;
+  while (true) {
+    const long long most = o->cancel ? std::min<long long>(batch * unit, per_launch) : per_launch;
+    const int count = (int)std::min(most, total - enq);
+    if (count > 0) {
+      run(count);
+      enq += count;
+    }
+    const Ctl& c = ctl_poll(ctx);
+    if (c.done || (use_stop && c.stop)) return (pdeb200_status)c.status;
+    if (enq >= total) return PDEB200_ERR_NOT_CONVERGED;
+    if (o->cancel && *o->cancel) {
+      ctl_set_done(ctx, PDEB200_ERR_CANCELLED);
+      return PDEB200_ERR_CANCELLED;
+    }
+    batch = std::min(2 * batch, cap);
+  }
+}
+
 // One solver iteration captured once as a CUDA graph and replayed. `iterate`
 // must only enqueue kernels on ctx->stream (they all read the device control
 // block, so a replay after convergence is a no-op like a direct launch). The

@@ -7,6 +7,8 @@ batch and launch sizes, stopping inside a batch.
 Tolerance: a sweep is a contraction of the error, and each adds a few
 roundings (FMA contraction is the only difference), so after S sweeps the
 fields differ by at most about 10 S eps relative: 1e-11 for S <= 4500."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -240,3 +242,21 @@ def test_cluster_bicgstab_iteration_limit(oracle_mod, iterations):
     st, ref, rrep = oracle_mod.rs_solve(p, opt)
     assert rep.status == abi.ERR_NOT_CONVERGED and rep.iterations == rrep.iterations == iterations
     assert rel_l2(got, ref) <= 1e-9
+
+
+# A cancel flag is seen after the first sweeps (8) or iteration, on grids held by
+# a cluster and by launches; a flag that stays 0 changes no bit.
+@pytest.mark.parametrize("method, first", [(abi.JACOBI, 8), (abi.CG, 1), (abi.BICGSTAB, 1)])
+@pytest.mark.parametrize("dims", [(41, 38, 1), (700, 690, 1)])
+def test_cancel_is_seen_between_iterations(method, first, dims):
+    p = make(dims, faces="none")
+    p.c = 0.0
+    opt = default_options(method=method, max_iter=150, tol=1e-13)
+    ref, rref = solver.solve(p, opt, raise_on_error=False)
+    flag = ctypes.c_int32(0)
+    opt.cancel = ctypes.pointer(flag)
+    got, rep = solver.solve(p, opt, raise_on_error=False)
+    assert (rep.status, rep.iterations) == (rref.status, rref.iterations) and np.array_equal(got, ref)
+    flag.value = 1
+    _, rep = solver.solve(p, opt, raise_on_error=False)
+    assert rep.status == abi.ERR_CANCELLED and rep.iterations == first
