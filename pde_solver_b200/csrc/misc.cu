@@ -476,14 +476,14 @@ pdeb200_status project_dev(Context* ctx, int nx, int ny, int nz, double dx, doub
     // 500x450 81 -> 39 ms
     CgProj pj{1.0 / (dx * dx), 1.0 / (dy * dy), g.is3 ? 1.0 / (dz * dz) : 0.0, 0.0, pin};
     pj.cc = -2.0 * (pj.cx + pj.cy + pj.cz);
-    const ClusterCgArgs a{dp, r, pc, ap, kClusterCgIters, nx, ny, g.nz, 0, n};
+    ClusterCgArgs a{dp, r, pc, ap, 0, nx, ny, g.nz, 0, n};
     auto kern = g.is3 ? cluster_cg_kernel<kCgProj3, CoefConst>(cs) : cluster_cg_kernel<kCgProj2, CoefConst>(cs);
-    auto run = [&](int) {
+    auto run = [&](int iters) {
+      a.iters = iters;
       launch_cluster(ctx, cs.csize, cs.threads, cs.smem, kern, GridDev{}, CoefConst{}, pj, a, C);
       ctx->count();
     };
-    o.check_interval = 1;
-    st = drive(ctx, &o, po->max_iter / kClusterCgIters + 1, run, false);
+    st = drive_runs(ctx, &o, po->max_iter + 1LL, 1, kClusterCgIters, run, false);
   } else {
     auto iterate = [&](int) {
       if (!g.is3) {

@@ -215,6 +215,20 @@ def test_cluster_projection_sizes(oracle_mod, dims):
         assert rel_l2(g, r) <= 1e-8
 
 
+# A negative limit makes no iteration.
+@pytest.mark.parametrize("max_iter", [-3, -1])
+@pytest.mark.parametrize("dims", [(33, 60, 1), (17, 16, 15)])
+def test_cluster_projection_iteration_limit(oracle_mod, dims, max_iter):
+    nx, ny, nz = dims
+    rng = np.random.Generator(np.random.PCG64(ny))
+    u, v, w, p = rng.standard_normal((4, nx * ny * nz))
+    a = (u, v, w if nz > 1 else None, p, nx, ny, nz, 0.02, 0.03, 0.025, 0.01, max_iter, 1e-30)
+    ug, vg, _, pg, rep = solver.project_velocity(*a)
+    _, ur, vr, _, pr, rrep = oracle_mod.rs_project(*a)
+    assert (rep.success, rep.poisson_iterations) == (rrep.success, rrep.poisson_iterations)
+    assert rel_l2(ug, ur) <= 1e-12 and rel_l2(vg, vr) <= 1e-12 and rel_l2(pg, pr) <= 1e-12
+
+
 # One and several virtual blocks and rounds; the 3D grid is served by launches. Both sides stop at a true residual of 1e-9 |b|, so the fields differ by
 # at most 2e-9 times the condition number, about (n / 2)^2 in n nodes a side.
 @pytest.mark.parametrize("dims", [(3, 3, 1), (3, 50, 1), (6, 40, 1), (40, 6, 1), (97, 81, 1), (161, 150, 1),
