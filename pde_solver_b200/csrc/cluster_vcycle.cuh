@@ -503,11 +503,14 @@ __device__ __forceinline__ bool cv_cycle(const unsigned char* __restrict__ image
     const CvGeo& c = geo[l + 1];
     const bool is3 = h.is3;
     if (h.work) {
-      // the coarse layers around this slab, boundary extension applied, in the
-      // residual's place (free by now) where they fit there
-      T* stage = Rr(l);
+      // the coarse layers around this slab, boundary extension applied (in FP64: in
+      // FP32 its factors' products would be rounded), in the residual's place (free
+      // by now) where they fit there. FP32 levels: 65^3 1.855 -> 1.875 ms per mixed
+      // solve against products rounded to FP32; applying the factors as the layers
+      // are read 1.92, no staging 1.95.
+      double* stage = reinterpret_cast<double*>(Rr(l));
       const int first = h.lo >> 1, layers = ((h.lo + h.n) >> 1) - first + 1;  // nested: coarse layers first ..
-      const bool staged = q.nested && layers * c.L <= q.nmax * q.L && h.n > 0;
+      const bool staged = q.nested && layers * c.L * sizeof(double) <= q.nmax * q.L * sizeof(T) && h.n > 0;
       if (staged) {
         for (int t = tid; t < layers * c.L; t += blockDim.x) {
           const int ly = cv_div(t, c.inv_L), in = t - ly * c.L, row = is3 ? cv_div(in, c.inv_nx) : 0;
@@ -520,7 +523,7 @@ __device__ __forceinline__ bool cv_cycle(const unsigned char* __restrict__ image
           cv_owner(c, ext_clamp(S, nl), o, pl);
           const T* src = cl_remote(X(l + 1), (unsigned)o) + pl * c.L + (is3 ? ext_clamp(row, c.ny) * c.nx : 0) +
                          ext_clamp(I, c.nx);
-          stage[t] = T(a * double(*src));
+          stage[t] = a * double(*src);
         }
         __syncthreads();
       }
@@ -540,15 +543,15 @@ __device__ __forceinline__ bool cv_cycle(const unsigned char* __restrict__ image
           double v;
           if (staged) {
             // mean of the two coarse nodes around the node on each axis (the same one twice on it)
-            const T* a0 = stage + ((s >> 1) - first) * c.L + (i >> 1);
-            const T* a1 = stage + (((s + 1) >> 1) - first) * c.L + (i >> 1);
+            const double* a0 = stage + ((s >> 1) - first) * c.L + (i >> 1);
+            const double* a1 = stage + (((s + 1) >> 1) - first) * c.L + (i >> 1);
             const int d = i & 1;
             if (is3) {
               const int r0 = (row >> 1) * c.nx, r1 = ((row + 1) >> 1) * c.nx;
-              v = 0.125 * (((double(a0[r0]) + double(a0[r0 + d])) + (double(a0[r1]) + double(a0[r1 + d]))) +
-                           ((double(a1[r0]) + double(a1[r0 + d])) + (double(a1[r1]) + double(a1[r1 + d]))));
+              v = 0.125 * (((a0[r0] + a0[r0 + d]) + (a0[r1] + a0[r1 + d])) +
+                           ((a1[r0] + a1[r0 + d]) + (a1[r1] + a1[r1 + d])));
             } else {
-              v = 0.25 * ((double(a0[0]) + double(a0[d])) + (double(a1[0]) + double(a1[d])));
+              v = 0.25 * ((a0[0] + a0[d]) + (a1[0] + a1[d]));
             }
           } else {
             const int j = is3 ? row : s;
