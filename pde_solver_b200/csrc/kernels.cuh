@@ -1051,12 +1051,6 @@ __device__ __forceinline__ double ext_axis(const ExtCoef& e, int a, int I, int n
 }
 __device__ __forceinline__ int ext_clamp(int I, int n) { return I < 1 ? 1 : (I > n - 2 ? n - 2 : I); }
 
-// The node-by-node form behind the scalar one (ARR instantiations), out of line.
-template <typename TC>
-__device__ __noinline__ double ext_value_arr(const GridDev& gc, const TC* __restrict__ xc, int I, int J, int K) {
-  return ext_value(gc, xc, I, J, K);
-}
-
 // Prolongation-add for any level pair: trilinear (bilinear in 2D)
 // interpolation of the coarse correction, extended to the coarse boundary
 // through the closures, added to the fine interior. A thread owns a fine
@@ -1088,13 +1082,14 @@ __global__ void __launch_bounds__(kBx* kBy) k_prolong(LevelGeo gf, LevelGeo gc, 
   const double w00 = ay0 * ax0, w10 = ay0 * ax1, w01 = ay1 * ax0, w11 = ay1 * ax1;
   const int cx0 = ext_clamp(I0, gc.nx), cx1 = ext_clamp(I1, gc.nx);
   const int cy0 = ext_clamp(J0, gc.ny) * gc.nx, cy1 = ext_clamp(J1, gc.ny) * gc.nx;
+  const bool xy_edge = I0 == 0 || I1 == gc.nx - 1 || J0 == 0 || J1 == gc.ny - 1;
   auto bilinear = [&](int K) -> double {
     double c00, c10, c01, c11;
-    if constexpr (ARR) {
-      c00 = ext_value_arr(gcf, xc, I0, J0, K);
-      c10 = ext_value_arr(gcf, xc, I1, J0, K);
-      c01 = ext_value_arr(gcf, xc, I0, J1, K);
-      c11 = ext_value_arr(gcf, xc, I1, J1, K);
+    if (ARR && (xy_edge || (is3 && (K == 0 || K == gc.nz - 1)))) {
+      c00 = ext_value(gcf, xc, I0, J0, K);
+      c10 = ext_value(gcf, xc, I1, J0, K);
+      c01 = ext_value(gcf, xc, I0, J1, K);
+      c11 = ext_value(gcf, xc, I1, J1, K);
     } else {
       const double az = is3 ? ext_axis(e, 2, K, gc.nz) : 1.0;
       const TC* p = xc + (is3 ? (long long)ext_clamp(K, gc.nz) * gc.sxy : 0);
@@ -1178,11 +1173,11 @@ __global__ void __launch_bounds__(kBx* kBy) k_prolong_pair(LevelGeo gf, LevelGeo
   // values through the closures, as in k_prolong)
   auto bil4 = [&](int K, double (&y)[4]) {
     double C00, C10, C01, C11;
-    if constexpr (ARR) {
-      C00 = ext_value_arr(gcf, xc, I, J, K);
-      C10 = ext_value_arr(gcf, xc, I + 1, J, K);
-      C01 = ext_value_arr(gcf, xc, I, J + 1, K);
-      C11 = ext_value_arr(gcf, xc, I + 1, J + 1, K);
+    if (ARR && (xy_edge || K == 0 || K == gc.nz - 1)) {
+      C00 = ext_value(gcf, xc, I, J, K);
+      C10 = ext_value(gcf, xc, I + 1, J, K);
+      C01 = ext_value(gcf, xc, I, J + 1, K);
+      C11 = ext_value(gcf, xc, I + 1, J + 1, K);
     } else {
       const TC* p = xc + (long long)ext_clamp(K, gc.nz) * gc.sxy;
       C00 = double(p[cy0 + cx0]);
