@@ -649,9 +649,10 @@ struct Hierarchy {
   // Levels from cv_l0 down run inside one cluster (k_cluster_vcycle): the
   // first level whose arrays, with those of the levels below, fit in the
   // shared memory of its CTAs (about 33^3 in FP64, 45k nodes in 2D). Not
-  // used when a coarse Neumann/Robin face has per-node closure factors (the
-  // transfer tables are per axis) or the coarsest level has more than
-  // kCvMaxCoarse interior nodes; the single-block tail serves those.
+  // used when the coarsest level has more than kCvMaxCoarse interior nodes, nor
+  // where coarse Neumann/Robin faces have per-node closure factors (the
+  // transfer tables are per axis) and so leave it fewer levels than the
+  // single-block tail, which serves those.
   int cv_l0 = -1;
   int cv_csize = 1, cv_coarse = 0;
   CvLayout cv_layout_;
@@ -682,7 +683,16 @@ struct Hierarchy {
       for (int a = 0; a < 3; ++a) levels[m].rt[a] = on[m] ? d + off[3 * m + a] : nullptr;
   }
 
-  void build_cluster(Context* ctx) {
+  // The first level of at most kTailMaxNodes nodes with at most kTailMaxLevels
+  // levels from it down, -1: none.
+  int first_tail_level() const {
+    for (size_t l = 0; l < levels.size(); ++l)
+      if (levels[l].g.n <= kTailMaxNodes && (int)(levels.size() - l) <= kTailMaxLevels) return (int)l;
+    return -1;
+  }
+
+  // last: the last level that may be the cluster's first
+  void build_cluster(Context* ctx, int last) {
     cv_l0 = -1;
     const int n = (int)levels.size();
     const GridDev& gc = levels.back().g;
@@ -696,7 +706,7 @@ struct Hierarchy {
         break;
       }
     }
-    for (int l = first; l < n; ++l) {
+    for (int l = first; l <= last; ++l) {
       if (interior_dofs(levels[l].g) > 1e6) continue;
       std::vector<CvLevel<Coef, T>> cv(n - l);
       std::vector<GridDev> gs;
@@ -808,13 +818,10 @@ struct Hierarchy {
     // kTailMaxLevels levels below it (colour-pass form only)
     tail_l0 = -1;
     cv_l0 = -1;
-    if (!fused && std::getenv("PDEB200_NO_TAIL") == nullptr) build_cluster(ctx);
-    if (cv_l0 < 0 && !fused && std::getenv("PDEB200_NO_TAIL") == nullptr) {
-      for (size_t l = 0; l < levels.size(); ++l)
-        if (levels[l].g.n <= kTailMaxNodes && (int)(levels.size() - l) <= kTailMaxLevels) {
-          tail_l0 = (int)l;
-          break;
-        }
+    if (!fused && std::getenv("PDEB200_NO_TAIL") == nullptr) {
+      const int tail = first_tail_level();
+      build_cluster(ctx, tail >= 0 ? tail : (int)levels.size() - 1);
+      if (cv_l0 < 0) tail_l0 = tail;
     }
     if (tail_l0 >= 0) {
       std::vector<TailLevel<Coef, T>> tl;

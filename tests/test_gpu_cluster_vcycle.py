@@ -96,3 +96,37 @@ def test_cluster_levels_mixed_precision(oracle_mod, bf16, dims):
     st, ref, _ = oracle_mod.rs_solve(p, default_options(method=abi.MG_PCG, tol=1e-13, tol_mode=abi.TOL_RELATIVE,
                                                         max_iter=300))
     assert st == 0 and rel_l2(got, ref) <= 1e-8  # the bar of the mixed form
+
+
+def kernels_of(p, opt):
+    """Names of the kernels that a solve launched under the profiler, without their level."""
+    lib = abi.load()
+    lib.pdeb200_profile_enable(0, 1)
+    try:
+        solver.solve(p, opt, raise_on_error=False)
+        stats = (abi.KernelStat * 256)()
+        n = lib.pdeb200_profile_read(0, stats, 256)
+    finally:
+        lib.pdeb200_profile_enable(0, 0)
+    return {stats[q].name.decode().split("@")[0] for q in range(n)}
+
+
+# Robin faces with a value per node: the transfer tables do not hold them, and the
+# levels below about 1100 nodes run in one block as they did before there was a
+# cluster form. Levels through the cluster else.
+@pytest.mark.parametrize("dims", [(33, 33, 33), (100, 37, 1), (34, 20, 27), (65, 40, 5)])
+def test_levels_with_closures_per_node(monkeypatch, dims):
+    p = make(dims, "const", MIXED)
+    opt = default_options(method=abi.MG_PCG, tol=0.0, tol_mode=abi.TOL_RELATIVE, max_iter=2)
+    used = kernels_of(p, opt)
+    assert "cluster_vcycle" in used and "tail_vcycle" not in used
+    nx, ny, nz = dims
+    rng = np.random.Generator(np.random.PCG64(nx))
+    p.faces[2] = FaceBC(abi.BC_ROBIN, alpha=1.0, beta=0.5, gamma=0.1, alpha_arr=1.0 + rng.random(nx * nz))
+    p.faces[0] = FaceBC(abi.BC_ROBIN, alpha=1.0, beta=0.5, gamma=0.1, beta_arr=0.1 + rng.random(ny * nz))
+    used = kernels_of(p, opt)
+    assert "tail_vcycle" in used and "cluster_vcycle" not in used
+    a, ra = solver.solve(p, opt, raise_on_error=False)
+    monkeypatch.setenv("PDEB200_NO_TAIL", "1")
+    b, rb = solver.solve(p, opt, raise_on_error=False)
+    assert ra.iterations == rb.iterations and rel_l2(a, b) <= 1e-11
