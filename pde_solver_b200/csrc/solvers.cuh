@@ -322,10 +322,13 @@ struct StepGraph {
   int state = -1;  // -1 not tried, 0 direct, 1 replay
   long long launches = 0;
   explicit StepGraph(bool differs) : first_differs(differs) {}
-  // `first`: enqueues iteration `it` directly; `repeat`: the one to replay
+  // `first`: enqueues iteration `it` directly; `repeat`: the one to replay. The
+  // driver also enqueues the one after the last of max_iter, which does nothing:
+  // nothing is captured for that.
   template <class First, class Repeat>
-  void step(Context* ctx, long long n, int it, First&& first, Repeat&& repeat) {
-    if (state < 0 && it >= 2 && launches > kDirectLaunches && n <= kDirectNodes) state = graph.capture(ctx, repeat) ? 1 : 0;
+  void step(Context* ctx, long long n, int max_iter, int it, First&& first, Repeat&& repeat) {
+    if (state < 0 && it >= 2 && it < max_iter && launches > kDirectLaunches && n <= kDirectNodes)
+      state = graph.capture(ctx, repeat) ? 1 : 0;
     if (state == 1 && !(first_differs && it == 0)) {
       graph.launch(ctx);
       return;
