@@ -146,11 +146,16 @@ pdeb200_status time_series_dev(Context* ctx, DevProblem& P, const pdeb200_time_o
   fill_boundary(ctx, g, buf[0], nullptr);
   // grids whose slabs fit in the shared memory of a cluster (about 120k nodes
   // in 2D) run all steps between two frames in one launch: 257x257, 200 steps
-  // with 5 frames 2.14 -> 0.93 ms
+  // with 5 frames 2.14 -> 0.93 ms. The launch loads and stores the field, so it
+  // pays from a few steps on, more of them the larger the grid (48 steps, ms, one
+  // launch per step / one per so many steps: 97x65 1.35 / 1.65 with 1, 0.95 / 0.84
+  // with 2, 0.73 / 0.57 with 3; 374x267 with k 2.10 / 2.30 with 2, 1.02 / 1.04
+  // with 6, 0.69 / 0.64 with 16).
+  const int per_launch = cb ? std::min(stride, frames - 1) : frames - 1;
   const ClusterShape cs = cluster_shape(g, 1024, ctx->max_cluster);
   const size_t smem = (2 * sizeof(double)) * (size_t)cs.buf_nodes +
                       (sizeof(unsigned) + sizeof(double)) * (size_t)cs.cnt_max;
-  const bool clustered = cs.csize > 0 && smem <= kClusterDynSmem;
+  const bool clustered = cs.csize > 0 && smem <= kClusterDynSmem && per_launch >= 3 + n / 16384;
   Buf other;
   if (!clustered) {
     other = Buf(sizeof(double) * n, ctx->stream);

@@ -167,6 +167,27 @@ def test_time_series_frames_and_boundaries(oracle_mod, dims, faces):
     assert np.array_equal(got, seen[23])
 
 
+# The steps between two frames run one per launch or all in one, by their number
+# and the grid's size: the same bits.
+@pytest.mark.parametrize("dims", [(3, 3, 1), (70, 41, 1), (300, 200, 1), (3, 4, 5), (19, 18, 20)])
+@pytest.mark.parametrize("coef", ["const", "divk"])
+def test_time_series_frame_stride_changes_no_bit(dims, coef):
+    p = make(dims, coef)
+    p.ut = 1.0
+    p.u0 = np.random.Generator(np.random.PCG64(1)).standard_normal(p.n)
+    dt = 0.05 * min(1.0 / (d - 1) for d in dims if d > 1) ** 2
+    frames = {}
+    for stride in (1, 2, 3, 4, 8, 100):
+        seen = {}
+        got, rep = solver.time_series(p, 0.0, dt, 26, on_frame=lambda q, t, u: seen.__setitem__(q, u),
+                                      frame_stride=stride)
+        assert rep.iterations == 25 and sorted(seen) == sorted(set(range(0, 26, stride)) | {25})
+        frames = frames or seen
+        assert np.array_equal(got, frames[25])
+        for q, u in seen.items():
+            assert np.array_equal(u, frames[q])
+
+
 # Krylov loops: the grids are held in shared memory, then with x, r and q in
 # global memory, then by a launch per step. Both sides stop at the same
 # tolerance, so the fields agree to that tolerance times the operator's
