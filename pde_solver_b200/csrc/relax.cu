@@ -516,9 +516,13 @@ pdeb200_status gauss_seidel(Context* ctx, DevProblem& P, const Coef& cf, const p
   const unsigned long long budget = 60ULL * 1000000000ULL;  // device-time guard of the single-launch forms: 60 s
   const ClusterShape cs = cluster_shape(g, 512, ctx->max_cluster);
   const size_t lex_smem = sizeof(double) * (size_t)cs.buf_nodes + (sizeof(double) + sizeof(uint2)) * (size_t)cs.slots;
-  // grids whose slabs fit in the shared memory of a cluster (about 160k nodes
-  // in 2D): 97x65 SOR 483 -> 16.5 ms, and no grid is faster in the one-block form
-  if (cs.csize > 0 && lex_smem <= kClusterDynSmem) {
+  // Grids whose slabs fit in the shared memory of a cluster (about 160k nodes
+  // in 2D): 97x65 SOR 483 -> 16.5 ms. A sweep alone takes as many steps there as
+  // barriers in one block, and a step visits half of a CTA's nodes, so a run of
+  // few sweeps stays in one block (ms in one block / cluster: 97x65 with k 0.29 /
+  // 0.33 for 2 sweeps, 0.52 / 0.34 for 4; 374x267 with nodal coefficients 8.7 / 11.1
+  // for 8, 17.2 / 11.3 for 16; 2353x3 in one CTA 4.2 / 4.7 for 4, 8.2 / 4.7 for 8).
+  if (cs.csize > 0 && lex_smem <= kClusterDynSmem && max_iter >= 4 + cs.cnt_max / 512) {
     Buf save(sizeof(double) * (size_t)cs.buf_nodes * cs.csize, ctx->stream);
     ClusterLexArgs a{P.f, P.f_const, omega, o->tol, max_iter, cs.buf_nodes, cs.slots, save.as<double>(), budget};
     auto kern = g.dim == 3 ? (P.nl.n ? k_cluster_lex<3, Coef, true> : k_cluster_lex<3, Coef, false>)

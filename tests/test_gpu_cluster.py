@@ -92,6 +92,14 @@ def test_cluster_jacobi_last_delta_is_of_the_field(dims, sweeps):
     assert ra.last_delta == np.abs(a - b).reshape(shape)[inner].max()
 
 
+# Runs of few sweeps in one block, of more in a cluster (from 4 sweeps on, 7 or 8
+# on the larger grids).
+@pytest.mark.parametrize("dims", [(23, 18, 1), (97, 65, 1), (200, 180, 1), (20, 19, 35), (1200, 3, 1)])
+@pytest.mark.parametrize("sweeps", [3, 4, 5, 6, 7, 8, 9])
+def test_lexicographic_few_sweeps(oracle_mod, dims, sweeps):
+    check(oracle_mod, make(dims), method=abi.GAUSS_SEIDEL, max_iter=sweeps, tol=0.0)
+
+
 # A batch shorter than the one before it (the last before the sweep limit: 64,
 # 128 .. 512 sweeps, then 1 or 2): every warp takes the same branch after each
 # batch. One launch form only, so each run gives the same bits; against the
