@@ -475,6 +475,7 @@ pdeb200_status project_dev(Context* ctx, int nx, int ny, int nz, double dx, doub
   ctx->count(8);
   pdeb200_options o{};
   pdeb200_status st;
+  IterGraph graph;  // destroyed after the last launches, not between them
   const CgShape cs = cg_shape(nx, ny, g.nz, ctx->max_cluster);
   if (cs.csize > 0) {
     // the loop inside one cluster: 256x256 19.5 -> 4.9 us per iteration,
@@ -507,7 +508,6 @@ pdeb200_status project_dev(Context* ctx, int nx, int ny, int nz, double dx, doub
     };
     // the iteration is captured once as a CUDA graph and replayed (projection
     // sizes are launch-bound: 256^2 takes about 24 us per iteration as direct launches)
-    IterGraph graph;
     const bool graphed = graph.capture(ctx, iterate);
     auto step = [&](int it) {
       if (graphed)
