@@ -1112,8 +1112,8 @@ __global__ void __launch_bounds__(kBx* kBy) k_prolong(LevelGeo gf, LevelGeo gc, 
   const int zmode = map_mode(gf.nz, gc.nz);
   // coarse interval of plane k and its remainder, advanced without divisions
   const int m = gc.nz - 1, den = gf.nz - 1;
-  Kc = zmode == 0 ? k0 : (zmode == 1 ? k0 >> 1 : (k0 * m) / den);
-  int rem = k0 * m - Kc * den;
+  Kc = zmode == 0 ? k0 : (zmode == 1 ? k0 >> 1 : (int)((long long)k0 * m / den));
+  int rem = (int)((long long)k0 * m - (long long)Kc * den);
   double ya = bilinear(Kc), yb = bilinear(min(Kc + 1, gc.nz - 1));
   int Ka = Kc;  // ya, yb: planes Ka, Ka + 1
   constexpr int kGroup = 4;

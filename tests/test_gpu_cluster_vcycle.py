@@ -130,3 +130,19 @@ def test_levels_with_closures_per_node(monkeypatch, dims):
     monkeypatch.setenv("PDEB200_NO_TAIL", "1")
     b, rb = solver.solve(p, opt, raise_on_error=False)
     assert ra.iterations == rb.iterations and rel_l2(a, b) <= 1e-11
+
+
+# More than 65536 planes: a fine plane's number times the coarse intervals does not
+# fit in 32 bits. Nested and not nested, coarsened along z only; as many
+# iterations as on a grid where it does.
+@pytest.mark.parametrize("nz", [70000, 70001])
+def test_prolongation_of_many_planes(nz):
+    its = []
+    for planes in (nz, nz - 10000):
+        p = GridProblem(3, 3, planes, bounds=(0.0, 1.0, 0.0, 1.0, 0.0, planes / 2.0), a=-1.0, b=-1.0, az=-1.0, e=0.05)
+        p.f = np.random.Generator(np.random.PCG64(7)).standard_normal(p.n)
+        p.faces = [FaceBC.neumann(0.0)] * 4 + [FaceBC.dirichlet(0.0)] * 2
+        got, rep = solver.solve(p, default_options(method=abi.MG_PCG, tol=1e-10, tol_mode=abi.TOL_RELATIVE, max_iter=60))
+        assert rep.status == abi.OK and rep.rel_residual <= 1.1e-10
+        its.append(rep.iterations)
+    assert abs(its[0] - its[1]) <= 1 and its[0] <= 30
