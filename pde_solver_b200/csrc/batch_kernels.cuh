@@ -935,7 +935,9 @@ __global__ void __launch_bounds__(kBThreads, 5) kb_prolong(const BTile* __restri
         const int o01 = ty.i[1] * gc.nx + tx.i[0], o11 = ty.i[1] * gc.nx + tx.i[1];
         auto plane = [&](int K) -> A {
           const float* p = xc + (long long)K * gc.sxy;
-          return (w00 * A(p[o00]) + w10 * A(p[o10])) + (w01 * A(p[o01]) + w11 * A(p[o11]));
+          // (a weight of 0, of a coarse neighbour outside or a Dirichlet face, takes no value)
+          auto part = [](A w, float v) { return w == A(0) ? A(0) : w * A(v); };
+          return (part(w00, p[o00]) + part(w10, p[o10])) + (part(w01, p[o01]) + part(w11, p[o11]));
         };
         if (gf.dim != 3) {
           const long long id = bid(gf, i, j, 0);

@@ -523,7 +523,7 @@ __device__ __forceinline__ bool cv_cycle(const unsigned char* __restrict__ image
           cv_owner(c, ext_clamp(S, nl), o, pl);
           const T* src = cl_remote(X(l + 1), (unsigned)o) + pl * c.L + (is3 ? ext_clamp(row, c.ny) * c.nx : 0) +
                          ext_clamp(I, c.nx);
-          stage[t] = a * double(*src);
+          stage[t] = ext_scale(a, double(*src));
         }
         __syncthreads();
       }
@@ -579,7 +579,7 @@ __device__ __forceinline__ bool cv_cycle(const unsigned char* __restrict__ image
                   cv_owner(c, ty.i[bb], o, pl);
                   p = cl_remote(X(l + 1), (unsigned)o) + pl * c.L;
                 }
-                double rs = tx.w[0] * double(p[tx.i[0]]);
+                double rs = ext_scale(tx.w[0], double(p[tx.i[0]]));
                 if (tx.w[1] != 0.0) rs += tx.w[1] * double(p[tx.i[1]]);
                 sum += ty.w[bb] * rs;
               }

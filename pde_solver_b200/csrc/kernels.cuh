@@ -1049,6 +1049,8 @@ inline bool ext_coef(const GridDev& g, ExtCoef* e) {
 __device__ __forceinline__ double ext_axis(const ExtCoef& e, int a, int I, int n) {
   return I == 0 ? e.lo[a] : (I == n - 1 ? e.hi[a] : 1.0);
 }
+// A boundary value from its factor: 0 on a Dirichlet face, whatever the value beside it.
+__device__ __forceinline__ double ext_scale(double a, double v) { return a == 0.0 ? 0.0 : a * v; }
 __device__ __forceinline__ int ext_clamp(int I, int n) { return I < 1 ? 1 : (I > n - 2 ? n - 2 : I); }
 
 // Prolongation-add for any level pair: trilinear (bilinear in 2D)
@@ -1095,10 +1097,10 @@ __global__ void __launch_bounds__(kBx* kBy) k_prolong(LevelGeo gf, LevelGeo gc, 
       const TC* p = xc + (is3 ? (long long)ext_clamp(K, gc.nz) * gc.sxy : 0);
       const double v00 = double(p[cy0 + cx0]), v10 = double(p[cy0 + cx1]);
       const double v01 = double(p[cy1 + cx0]), v11 = double(p[cy1 + cx1]);
-      c00 = az * w00 * v00;
-      c10 = az * w10 * v10;
-      c01 = az * w01 * v01;
-      c11 = az * w11 * v11;
+      c00 = ext_scale(az * w00, v00);
+      c10 = ext_scale(az * w10, v10);
+      c01 = ext_scale(az * w01, v01);
+      c11 = ext_scale(az * w11, v11);
     }
     const double x0 = (1.0 - tx) * c00 + tx * c10, x1 = (1.0 - tx) * c01 + tx * c11;
     return (1.0 - ty) * x0 + ty * x1;
@@ -1186,10 +1188,10 @@ __global__ void __launch_bounds__(kBx* kBy) k_prolong_pair(LevelGeo gf, LevelGeo
       C11 = double(p[cy1 + cx1]);
       if (xy_edge || K == 0 || K == gc.nz - 1) {
         const double az = ext_axis(e, 2, K, gc.nz);
-        C00 *= az * (ay0 * ax0);
-        C10 *= az * (ay0 * ax1);
-        C01 *= az * (ay1 * ax0);
-        C11 *= az * (ay1 * ax1);
+        C00 = ext_scale(az * (ay0 * ax0), C00);
+        C10 = ext_scale(az * (ay0 * ax1), C10);
+        C01 = ext_scale(az * (ay1 * ax0), C01);
+        C11 = ext_scale(az * (ay1 * ax1), C11);
       }
     }
 #pragma unroll
