@@ -659,7 +659,7 @@ struct MgBicgCore {
       ctx->count(6);
     };
     // iterations after the first are identical
-    auto step = [&](int it) { graph.step(ctx, n, max_iter, it, iterate, [&](int) { iterate(1); }); };
+    auto step = [&](int it) { graph.step(ctx, n, H.cv_l0 >= 0, max_iter, it, iterate, [&](int) { iterate(1); }); };
     pdeb200_status st = drive(ctx, o, max_iter + 1, step, false);
     const Ctl c = ctl_poll(ctx);
     *iters = c.iter;
@@ -794,7 +794,7 @@ struct MgPcgCore {
       launch_dep(ctx, dim3(nb), dim3(256), 0, k_cg_p<T>, n, p, (const T*)z, (const Ctl*)C, 0);
       ctx->count(3);
     };
-    auto step = [&](int it) { graph.step(ctx, n, max_iter, it, iterate, iterate); };
+    auto step = [&](int it) { graph.step(ctx, n, H.cv_l0 >= 0, max_iter, it, iterate, iterate); };
     pdeb200_status st = drive(ctx, o, max_iter + 1, step, false);
     const Ctl c = ctl_poll(ctx);
     *iters = c.iter;

@@ -228,7 +228,7 @@ pdeb200_status mg_pcg(Context* ctx, DevProblem& P, const Coef& cf, const pdeb200
     ctx->count(2);
   };
   StepGraph graph{false};
-  auto step = [&](int it) { graph.step(ctx, n, max_iter, it, iterate, iterate); };
+  auto step = [&](int it) { graph.step(ctx, n, H.cv_l0 >= 0, max_iter, it, iterate, iterate); };
   // |r|^2 <= tol2 on the device (PostRRRel): batches sized by the observed reduction rate
   pdeb200_status st = drive(ctx, o, max_iter + 1, step, false, true);
   const Ctl c = ctl_poll(ctx);

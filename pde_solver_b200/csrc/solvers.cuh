@@ -312,9 +312,13 @@ struct IterGraph {
 // instantiation and destruction (0.5 ms) are not earned back: 257x193 1.72 ->
 // 1.52 ms with one memset for all levels. So do those of grids above
 // kDirectNodes, whose kernels take 5 us and more: 513^3 mixed BiCGStab 85.6 -> 84.3 ms.
+// Without a cluster kernel among them the launches are short, and a long solve
+// is captured all the same (from iteration kFewLaunchesFrom on, when its 0.4 ms
+// are earned back: 236x47 in two levels 65 -> 56 us per iteration, 5x200x6 62 -> 56).
 struct StepGraph {
   static constexpr long long kDirectLaunches = 24;
   static constexpr long long kDirectNodes = 1LL << 20;
+  static constexpr int kFewLaunchesFrom = 24;
   // iteration 0 of every solve starts otherwise than the replayed one (an
   // object that serves several solves launches each solve's first directly)
   const bool first_differs;
@@ -326,9 +330,9 @@ struct StepGraph {
   // driver also enqueues the one after the last of max_iter, which does nothing:
   // nothing is captured for that.
   template <class First, class Repeat>
-  void step(Context* ctx, long long n, int max_iter, int it, First&& first, Repeat&& repeat) {
-    if (state < 0 && it >= 2 && it < max_iter && launches > kDirectLaunches && n <= kDirectNodes)
-      state = graph.capture(ctx, repeat) ? 1 : 0;
+  void step(Context* ctx, long long n, bool cluster, int max_iter, int it, First&& first, Repeat&& repeat) {
+    const int from = launches > kDirectLaunches ? 2 : (cluster ? max_iter : kFewLaunchesFrom);
+    if (state < 0 && it >= from && it < max_iter && n <= kDirectNodes) state = graph.capture(ctx, repeat) ? 1 : 0;
     if (state == 1 && !(first_differs && it == 0)) {
       graph.launch(ctx);
       return;

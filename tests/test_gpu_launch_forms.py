@@ -83,3 +83,18 @@ def test_graph_replay_changes_no_numbers_in_refinement(monkeypatch, dims):
     b, rb = solver.solve(p, opt)
     assert ra.status == abi.OK and ra.iterations == rb.iterations and ra.iterations >= 6
     assert np.array_equal(a, b)
+
+
+def test_graph_replay_of_a_long_solve_of_few_launches(monkeypatch):
+    # two levels and closures per node: no cluster kernel, at most 24 launches per
+    # iteration, captured late
+    p = GridProblem(48, 54, 13, a=-1.0, b=-1.0, az=-1.0)
+    rng = np.random.Generator(np.random.PCG64(2))
+    p.f = rng.standard_normal(p.n)
+    p.faces[0] = FaceBC(abi.BC_ROBIN, alpha=1.5, beta=0.1, gamma=0.2, alpha_arr=1.0 + rng.random(54 * 13))
+    opt = default_options(method=abi.MG_PCG, tol=0.0, tol_mode=abi.TOL_RELATIVE, max_iter=45, mg_max_levels=2,
+                          mg_coarse_iters=1)
+    a, ra = solver.solve(p, opt, raise_on_error=False)
+    monkeypatch.setenv("PDEB200_NO_GRAPH", "1")
+    b, rb = solver.solve(p, opt, raise_on_error=False)
+    assert ra.iterations == rb.iterations == 45 and np.array_equal(a, b)
