@@ -3,15 +3,15 @@
 // A Jacobi sweep or a heat step of a small grid is a microsecond of work
 // behind two launches, and a lexicographic Gauss-Seidel sweep is one barrier
 // per hyperplane. Here up to 16 CTAs of one cluster hold the grid in their
-// shared memory and run many sweeps per launch, with one cluster barrier
-// (hardware, no spinning on memory) per step.
+// shared memory and run many sweeps per launch; the CTAs meet in each step by
+// their neighbours' copies (ClusterExchange), not by a barrier of all.
 //
 // The grid is cut into slabs of whole layers along its slowest dimension
 // (rows in 2D, planes in 3D). A CTA keeps its layers plus the layer before and
 // after them; the thread that updates a node of a slab's first or last layer
-// also stores the value into the neighbour CTA's copy (distributed shared
+// also sends the value to the neighbour CTA's copy (distributed shared
 // memory), and the thread that updates a node next to a face writes that
-// face's closure, so nothing but the barrier separates two sweeps.
+// face's closure, so nothing but the exchange separates two sweeps.
 #pragma once
 
 #include "../../include/pdeb200.h"
@@ -330,7 +330,9 @@ struct ClusterSweepArgs {
 // met the tolerance.
 //
 // Bound by latency: a warp issues one instruction of a node's dependent chain
-// about every five cycles. 129x129: 0.90 us per sweep in 16 CTAs against
+// about every five cycles (129x129: half of the issue slots of its SMs, of
+// 8 resident warps' wait per issue 2.5 on the chain, 1.5 on shared memory, 1.0 at
+// the block barrier). 129x129: 0.90 us per sweep in 16 CTAs against
 // 7.5 us as two launches in a replayed graph (22392 sweeps 168 -> 20.2 ms); with
 // a releasing cluster barrier per sweep and the test in every warp 1.4 us.
 template <int D, class Coef, bool HEAT, bool NL>

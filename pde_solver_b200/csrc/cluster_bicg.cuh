@@ -44,8 +44,9 @@ constexpr size_t kBiSmem = sizeof(double) * 5 * kBiThreads * kBiRounds;
 
 // Iterations from x, r, p, v and the scalars of ctl to the stopping test or
 // a.iters; the field ends in a.x. Bound by latency: 97x81 with per-node
-// coefficients 13.4 us per iteration (five phases of two L2 round trips and a releasing cluster barrier) against 43 us
-// as launches; sums in another order (3 phases) would stop at another iteration.
+// coefficients 13 to 20 us per iteration from GPU to GPU (five phases of two L2
+// round trips and a releasing cluster barrier; per issue 11.5 warps wait at
+// barriers, 3.9 for the fences, 3.8 for L2) against 43 to 62 us as launches; sums in another order (3 phases) would stop at another iteration.
 template <class Coef>
 __global__ void __launch_bounds__(kBiThreads) k_cluster_bicg(GridDev g, Coef cf, ClusterBicgArgs a, Ctl* ctl) {
   extern __shared__ double wts[];  // folded into rounds: weights c, xp, xm, yp, ym of this thread's nodes

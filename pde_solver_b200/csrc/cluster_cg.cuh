@@ -71,7 +71,8 @@ inline CgShape cg_shape(int nx, int ny, int nz, int most) {
 // (L2).
 // At 256x256 (4096 nodes per CTA) an iteration takes 4.9 us against 19.5 us as
 // four launches of a replayed graph: about half of it shared-memory bandwidth
-// (33 wavefronts per 32 nodes), 1.2 us the two sums. Measured slower there:
+// (33 wavefronts per 32 nodes), 1.2 us the two sums (the SMs issue in 30% of their
+// cycles; per issue 4.7 warps wait at barriers, 4.4 for shared memory). Measured slower there:
 // 992 threads (5.5 us), x, r, q and p in registers (6.8 us, spills at 8 nodes a
 // thread), padded rows with wall cells and an offset table (5.4 us).
 template <int OP, class Coef, bool SM>

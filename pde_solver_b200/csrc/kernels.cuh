@@ -1345,7 +1345,7 @@ __global__ void k_coarse_solve_smem(GridDev g, Coef cf, const TB* __restrict__ b
 // prolongation-add of the extended correction and `post` sweeps (colour order
 // reversed), and `coarse_iters` sweeps from zero on the coarsest level. The
 // arithmetic of every node update is that of k_rbgs / k_residual_folded /
-// full_weight / k_restrict_fold_faces / k_prolong_add. rhs0 is the right-hand side of
+// full_weight / k_restrict_fold_faces / k_prolong. rhs0 is the right-hand side of
 // level 0 of the tail; the result is left in lv[0].x.
 template <class Coef, typename T>
 struct TailLevel {

@@ -95,8 +95,8 @@ __device__ __forceinline__ void fe_close(const GridDev& g, double* next, long lo
 // and the Neumann/Robin closures at t+dt, each written by the thread of the
 // node next to the face (Dirichlet values are in both buffers; edges and
 // corners, which no step reads, are filled when a frame is handed out). With
-// the closures as a launch of their own a step of a small grid cost two
-// launches: FENUM
+// the closures as a launch of their own a step took two launches: 60x50x40, 48
+// steps 1.22 -> 0.56 ms.
 template <class Coef>
 __global__ void __launch_bounds__(kBx* kBy) k_fe_step(GridDev g, Coef cf, const double* __restrict__ f, double fc,
                                                       NonlinDev nl, double ut, double dt, const double* __restrict__ u,

@@ -415,6 +415,8 @@ __global__ void __launch_bounds__(32 * S::W, S::kMinBlocks)
 // 165 at the copy rate), residual 305 (371, 250); with the sums 380, where the
 // separate dot products take another 130 to 165. FP64 300^3: 95 (111), residual no
 // faster (121, 120), so that keeps k_residual_folded.
+// Warps per block, rows per lane: the 513^3 mixed solve 61.0 ms with 4 x 4, 62.5 with
+// 2 warps, 61.3 with 8, 63.2 with 2 rows, 62.4 with 6.
 constexpr int kColW = 4, kColRows = 4;
 // planes per block: without a sum short chunks spread the work, with one fewer
 // blocks leave fewer partial sums (513^3 FP32 21 / 43 / 86 planes: apply 238 / 242 /
